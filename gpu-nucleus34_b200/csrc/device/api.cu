@@ -315,6 +315,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	r.variant = variant;
 	Incidence inc;
 	CliqueCsr csr;
+	BitMats mats;
 	int32_t *S = nullptr;
 	uint32_t *own = nullptr;
 	int rc = NUCLEUS34_OK;
@@ -324,7 +325,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	{
 		c.peel_debit_sec = 0;
 		N34_CUDA(cudaEventRecord(ev.e[0], c.stream));
-		if ((rc = list_triangles(c)))
+		if ((rc = list_triangles(c, bit_form_wanted(c, variant) ? &mats : nullptr)))
 			break;
 		if ((rc = segments_after_listing(c)))
 			break;
@@ -341,7 +342,18 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 			break;
 		}
 		c.lean_run = false;
-		if (c.T)
+		// the on-demand variant runs on the listing's bit matrices when they
+		// were kept and the rest fits beside them, else on the incidence lists
+		const bool bits = c.T && bit_form_fits(c, mats);
+		if (!bits)
+			free_mats(c, mats);
+		if (bits)
+		{
+			if ((rc = build_in_lists(c, mats, inc)))
+				break;
+			r.sum_te_sq = inc.sum_te_sq;
+		}
+		else if (c.T)
 		{
 			// The on-demand peel with death flags (T < 2^30) uses either the
 			// regular layout (64-bit sort keys beside the entries, each
@@ -369,7 +381,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (variant == NUCLEUS34_DIRECT && (rc = dalloc(c, &own, c.T, "clique owner counts")))
 				break;
-			if ((rc = count_support(c, inc, S, &total, own)))
+			if ((rc = bits ? count_support_bits(c, mats, inc, S, &total) : count_support(c, inc, S, &total, own)))
 				break;
 			if (total % 4)
 			{
@@ -418,7 +430,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (total)
 			{
-				if ((rc = peel(c, variant, inc, csr, S, c.dK, &pc)))
+				if ((rc = bits ? peel_bits(c, mats, inc, S, c.dK, &pc) : peel(c, variant, inc, csr, S, c.dK, &pc)))
 					break;
 				peeled = true;
 			}
@@ -434,6 +446,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	} while (false);
 	free_incidence(c, inc);
 	free_clique_csr(c, csr);
+	free_mats(c, mats);
 	c.release(S);
 	c.release(own);
 	if (rc)

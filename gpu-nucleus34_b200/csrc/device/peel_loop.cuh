@@ -1,0 +1,598 @@
+// The level-synchronous peel as one cooperative launch.
+//
+// All blocks of the launch are resident at once and run every round of the
+// peel, phases separated by grid barriers; nothing is launched and no size is
+// read by the host in between. A round is two phases:
+//   mark    the frontier's triangles get their k and their death stamp (the
+//           support word becomes 0x80000000 | round); the frontier before it
+//           is retired (what a path keeps per dead triangle is cleared)
+//   debit   every dying triangle enumerates its live four-cliques and debits
+//           the partners still alive; a partner that falls to the level is
+//           appended to the next frontier
+// An empty next frontier is a level change: one more phase scans the supports
+// for the triangles at level + 1 (and the minimum, should none sit there). A
+// large next frontier is put in id order through a bitmap (two phases), so
+// that neighbouring warps work on triangles that share their rows and lists.
+//
+// Round-to-round cost is what bounds the small graphs and the long tails of
+// the large ones: with every step of a round a kernel of its own (13 launches
+// in a CUDA graph's while node) a round took 38 us on R-MAT scale 12 and 66 us
+// on scale 16, with most of the launches empty; here it takes 14 and 40 us.
+//
+// The counters that a phase fills (appended triangles, minimum support) live
+// in one of four slots taken in turn; every block reads the slot right after
+// the phase's barrier, and it is cleared two phases later, when no block can
+// still read it.
+#pragma once
+
+#include <algorithm>
+
+#include "common.cuh"
+
+namespace n34 {
+
+// Two blocks of 512 threads per SM, 64 registers each (three blocks of 40
+// registers: 13% slower on R-MAT scale 18; one of 1024: 2% slower).
+constexpr uint32_t LOOP_THREADS = 512;
+constexpr uint32_t LOOP_WARPS = LOOP_THREADS / 32;
+constexpr uint32_t NO_SUPPORT = 0xffffffffu;
+// A barrier wait longer than this ends the launch (every block leaves at its
+// next barrier and the call returns E_TIMEOUT); so does a peel longer than
+// LOOP_TIME_LIMIT_NS. R-MAT scale 20 peels in about a second.
+constexpr unsigned long long LOOP_WAIT_LIMIT_NS = 60ull * 1000000000ull;
+constexpr unsigned long long LOOP_TIME_LIMIT_NS = 600ull * 1000000000ull;
+
+struct PhaseSlot
+{
+	uint32_t n;    // triangles appended in the phase
+	uint32_t mn;   // least support above the gathered level (scan phase)
+	uint32_t work; // units of the debit phase claimed beyond the first of each warp
+	uint32_t pad;
+};
+
+struct LoopCtl
+{
+	PeelCtl c; // results: peeled, ksum, kmax, rounds, error
+	uint32_t timed_out;
+	uint32_t arrived; // barrier arrivals, never reset (compared modulo 2^32)
+	uint32_t abort;
+	uint32_t scans, ordered;
+	PhaseSlot slot[4];
+	unsigned long long ns[4]; // time per phase kind: mark, debit, scan, order
+};
+
+struct LoopArgs
+{
+	LoopCtl *ctl;
+	int32_t *S;
+	int32_t *K;
+	uint32_t *R; // death rounds kept for the certificate, or null
+	uint32_t *F0, *F1;
+	uint32_t *fbits; // T bits, all zero (null: frontiers keep their order)
+	uint64_t T;
+	uint32_t sort_min; // frontiers at least this large are put in id order
+};
+
+__device__ __forceinline__ unsigned long long loop_ns()
+{
+	unsigned long long t;
+	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+	return t;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
+{
+	uint32_t v;
+	asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+	return v;
+}
+
+// A support word: weak load. Its sign and stamp only change in the mark phase;
+// debits of the running phase change the value of a live one alone.
+__device__ __forceinline__ int32_t ld_support(const int32_t *p)
+{
+	int32_t v;
+	asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+	return v;
+}
+
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
+{
+	const uint32_t lane = lane_id();
+#pragma unroll
+	for (uint32_t o = 1; o < 32; o <<= 1)
+	{
+		const uint32_t y = __shfl_up_sync(FULL, v, o);
+		if (lane >= o)
+			v += y;
+	}
+	return v;
+}
+
+// First lane whose inclusive sum exceeds k (31 if none): the lane that item k
+// of the warp's concatenated items belongs to.
+__device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t k)
+{
+	uint32_t s = 0;
+#pragma unroll
+	for (uint32_t step = 16; step > 0; step >>= 1)
+		if (__shfl_sync(FULL, incl, s + step - 1) <= k)
+			s += step;
+	return s;
+}
+
+// Position of the r-th (from 0) set bit of z; r < popc(z).
+__device__ __forceinline__ uint32_t nth_bit(uint32_t z, uint32_t r)
+{
+	uint32_t pos = 0;
+#pragma unroll
+	for (uint32_t w = 16; w > 0; w >>= 1)
+	{
+		const uint32_t c = __popc(z & ((1u << w) - 1u));
+		if (r >= c)
+		{
+			r -= c;
+			z >>= w;
+			pos += w;
+		}
+	}
+	return pos;
+}
+
+// A warp's triangles for the next frontier, collected in shared memory and
+// handed over many at a time: atomics of all warps on the one counter of the
+// frontier take about 5.5 cycles each (2.8 ns, whole GPU), which bounded the
+// debit when every step with a crossing appended by itself (peel of the random
+// geometric graph with 500k points: 106 ms, 69 with the buffer; R-MAT scale 18:
+// 265 and 233 ms).
+struct Appender
+{
+	static constexpr uint32_t CAP = 128;
+	uint32_t *buf;  // CAP entries of this warp
+	uint32_t *Fn;   // next frontier
+	uint32_t *n;    // its size
+	uint32_t *err;
+	uint64_t T;     // capacity
+	uint32_t count; // entries in buf (warp-uniform)
+
+	// t for the lanes with hit set (all lanes call)
+	__device__ __forceinline__ void push(bool hit, uint32_t t)
+	{
+		const uint32_t m = __ballot_sync(FULL, hit);
+		if (hit)
+			buf[count + __popc(m & lanemask_lt())] = t;
+		count += __popc(m);
+	}
+	// makes room for three pushes (all lanes call)
+	__device__ __forceinline__ void drain()
+	{
+		if (count <= CAP - 96)
+			return;
+		__syncwarp();
+		uint32_t base = 0;
+		if (lane_id() == 0)
+			base = atomicAdd(n, count);
+		write(__shfl_sync(FULL, base, 0));
+	}
+	__device__ __forceinline__ void write(uint32_t base)
+	{
+		for (uint32_t i = lane_id(); i < count; i += 32)
+		{
+			if (uint64_t(base) + i < T)
+				Fn[base + i] = buf[i];
+			else
+				atomicOr(err, 1u);
+		}
+		__syncwarp();
+		count = 0;
+	}
+	// the rest of all warps of the block, with one atomic (all threads call)
+	__device__ __forceinline__ void finish()
+	{
+		__shared__ uint32_t s_at[LOOP_WARPS];
+		if (lane_id() == 0)
+			s_at[threadIdx.x >> 5] = count;
+		__syncthreads();
+		if (threadIdx.x < 32)
+		{
+			const uint32_t c = threadIdx.x < LOOP_WARPS ? s_at[threadIdx.x] : 0u;
+			const uint32_t x = warp_incl_scan(c);
+			uint32_t base = 0;
+			if (threadIdx.x == 31 && x)
+				base = atomicAdd(n, x);
+			base = __shfl_sync(FULL, base, 31);
+			if (threadIdx.x < LOOP_WARPS)
+				s_at[threadIdx.x] = base + x - c;
+		}
+		__syncthreads();
+		write(s_at[threadIdx.x >> 5]);
+	}
+};
+
+// Ownership of a clique among the members that die this round: the lowest id
+// (debit_partners' rule, cuNucleus34_ondemand.cu:237-276). True when dying
+// triangle t does not own it on account of a partner with support word s:
+// the partner died in an earlier round, or dies in this one with a lower id.
+__device__ __forceinline__ bool partner_blocks(int32_t s, uint32_t id, uint32_t t, uint32_t stamp)
+{
+	return s < 0 && (uint32_t(s) != stamp || id < t);
+}
+
+// How a debit phase is cut into units, which the warps claim as they go (the
+// first by their number, the others from the slot's counter): batches of ch
+// consecutive frontier triangles, at least sixteen per warp (a fixed stride
+// over two per warp took 325 ms of debit on R-MAT scale 18, claimed units of
+// that size 247); or, where the frontier has at most half as many triangles as
+// there are warps, one triangle shared by 2^shift warps (twice or four times as
+// many warps per triangle: 17% and 35% slower on R-MAT scale 12).
+struct Units
+{
+	uint32_t ch, total;
+	uint32_t shift; // log2 of the warps that share a triangle
+};
+
+__device__ __forceinline__ Units debit_units(uint32_t nF, uint32_t nwarps)
+{
+	Units u{1u, 0u, 0u};
+	while (u.ch < 32 && uint64_t(u.ch) * 16 * nwarps <= nF)
+		u.ch <<= 1;
+	while (u.shift < 6 && (nF << (u.shift + 1)) <= nwarps)
+		++u.shift;
+	u.total = ((nF + u.ch - 1) / u.ch) << u.shift;
+	return u;
+}
+
+// f(unit) for every unit of the phase (all lanes call f together).
+template <class Fn>
+__device__ __forceinline__ void claim_units(uint32_t total, uint32_t *work, Fn &&f)
+{
+	const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+	const uint32_t grab = min(max(total / (nwarps * 8), 1u), 16u); // units per claim
+	for (uint32_t unit = warp * grab; unit < total;)
+	{
+		uint32_t next = total;
+		if (total > nwarps * grab && lane_id() == 0)
+			next = nwarps * grab + atomicAdd(work, grab); // its latency is hidden by f
+		const uint32_t end = min(unit + grab, total);
+		for (; unit < end; ++unit)
+			f(unit);
+		unit = __shfl_sync(FULL, next, 0);
+	}
+}
+
+// End of a phase: grid barrier, then the phase's slot. False: leave.
+__device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_t &target, uint32_t &n, uint32_t &mn)
+{
+	__shared__ uint32_t s_n, s_mn, s_ok;
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		if (blockIdx.x == 0)
+			ctl->slot[(phase + 2) & 3] = PhaseSlot{0u, NO_SUPPORT, 0u, 0u};
+		__threadfence();
+		target += gridDim.x;
+		atomicAdd(&ctl->arrived, 1u);
+		uint32_t spins = 0;
+		unsigned long long t0 = 0;
+		while (int32_t(ld_acquire(&ctl->arrived) - target) < 0)
+		{
+			if ((++spins & 1023u) == 0)
+			{
+				if (__ldcg(&ctl->abort))
+					break;
+				const unsigned long long now = loop_ns();
+				if (!t0)
+					t0 = now;
+				else if (now - t0 > LOOP_WAIT_LIMIT_NS)
+					atomicExch(&ctl->abort, 1u);
+			}
+		}
+		__threadfence();
+		s_n = __ldcg(&ctl->slot[phase & 3].n);
+		s_mn = __ldcg(&ctl->slot[phase & 3].mn);
+		s_ok = __ldcg(&ctl->abort) == 0;
+	}
+	__syncthreads();
+	++phase;
+	n = s_n;
+	mn = s_mn;
+	return s_ok != 0;
+}
+
+// Appends every live triangle with support <= hi to F and takes the minimum of
+// the others. A warp reads 1024 supports per step, eight per thread at a time
+// (two 16-byte loads), and appends them with one atomic.
+__device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint32_t *__restrict__ F, PhaseSlot *slot)
+{
+	const uint32_t lane = lane_id();
+	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+	const uint64_t stride = ((uint64_t(gridDim.x) * blockDim.x) >> 5) * 1024;
+	uint32_t mn = NO_SUPPORT;
+	for (uint64_t b0 = warp * 1024; b0 < g.T; b0 += stride)
+	{
+		uint32_t mask = 0; // bit 8c + j: support j of this lane's chunk c
+#pragma unroll
+		for (uint32_t c = 0; c < 4; ++c)
+		{
+			const uint64_t t0 = b0 + c * 256 + lane * 8;
+			int32_t v[8];
+			if (t0 + 8 <= g.T)
+			{
+				const int4 a = *reinterpret_cast<const int4 *>(g.S + t0);
+				const int4 b = *reinterpret_cast<const int4 *>(g.S + t0 + 4);
+				v[0] = a.x;
+				v[1] = a.y;
+				v[2] = a.z;
+				v[3] = a.w;
+				v[4] = b.x;
+				v[5] = b.y;
+				v[6] = b.z;
+				v[7] = b.w;
+			}
+			else
+			{
+#pragma unroll
+				for (uint32_t j = 0; j < 8; ++j)
+					v[j] = t0 + j < g.T ? g.S[t0 + j] : -1;
+			}
+#pragma unroll
+			for (uint32_t j = 0; j < 8; ++j)
+				if (v[j] >= 0)
+				{
+					if (uint32_t(v[j]) <= hi)
+						mask |= 1u << (c * 8 + j);
+					else
+						mn = min(mn, uint32_t(v[j]));
+				}
+		}
+		if (!__ballot_sync(FULL, mask != 0))
+			continue;
+		uint32_t base = 0;
+		const uint32_t total = __shfl_sync(FULL, warp_incl_scan(__popc(mask)), 31);
+		if (lane == 0)
+			base = atomicAdd(&slot->n, total);
+		base = __shfl_sync(FULL, base, 0);
+#pragma unroll
+		for (uint32_t c = 0; c < 4; ++c)
+		{
+			uint32_t z = (mask >> (c * 8)) & 0xffu;
+			const uint32_t x = warp_incl_scan(__popc(z));
+			uint32_t pos = base + x - __popc(z);
+			while (z)
+			{
+				const uint32_t j = __ffs(z) - 1;
+				z &= z - 1;
+				if (pos < g.T)
+					F[pos] = uint32_t(b0 + c * 256 + lane * 8 + j);
+				else
+					atomicOr(&g.ctl->c.error, 1u);
+				++pos;
+			}
+			base += __shfl_sync(FULL, x, 31);
+		}
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		mn = min(mn, __shfl_xor_sync(FULL, mn, o));
+	if (lane == 0 && mn != NO_SUPPORT)
+		atomicMin(&slot->mn, mn);
+}
+
+// Order phase 1: the bits of F[0, n).
+__device__ __forceinline__ void order_set(const LoopArgs &g, const uint32_t *F, uint32_t n)
+{
+	const uint32_t stride = gridDim.x * blockDim.x;
+	for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+	{
+		const uint32_t t = F[i];
+		if (t < g.T)
+			atomicOr(g.fbits + (t >> 5), 1u << (t & 31));
+	}
+}
+
+// Order phase 2: the ids back to F, clearing the bits. A warp takes 128 words
+// (4096 ids) at a time, in id order inside and in the order the warps reach
+// them outside, which is close to id order.
+__device__ __forceinline__ void order_write(const LoopArgs &g, uint32_t *__restrict__ F, PhaseSlot *slot)
+{
+	const uint32_t lane = lane_id();
+	const uint64_t words = (g.T + 31) / 32;
+	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+	const uint64_t stride = ((uint64_t(gridDim.x) * blockDim.x) >> 5) * 128;
+	for (uint64_t w0 = warp * 128; w0 < words; w0 += stride)
+	{
+		uint32_t z[4], cnt = 0;
+#pragma unroll
+		for (uint32_t c = 0; c < 4; ++c)
+		{
+			const uint64_t w = w0 + c * 32 + lane;
+			z[c] = w < words ? g.fbits[w] : 0u;
+			cnt += __popc(z[c]);
+		}
+		if (!__ballot_sync(FULL, cnt != 0))
+			continue;
+		const uint32_t total = __shfl_sync(FULL, warp_incl_scan(cnt), 31);
+		uint32_t base = 0;
+		if (lane == 0)
+			base = atomicAdd(&slot->n, total);
+		base = __shfl_sync(FULL, base, 0);
+#pragma unroll
+		for (uint32_t c = 0; c < 4; ++c)
+		{
+			const uint64_t w = w0 + c * 32 + lane;
+			if (z[c])
+				g.fbits[w] = 0;
+			const uint32_t x = warp_incl_scan(__popc(z[c]));
+			uint32_t pos = base + x - __popc(z[c]);
+			while (z[c])
+			{
+				const uint32_t b = __ffs(z[c]) - 1;
+				z[c] &= z[c] - 1;
+				if (pos < g.T)
+					F[pos] = uint32_t(w * 32 + b);
+				++pos;
+			}
+			base += __shfl_sync(FULL, x, 31);
+		}
+	}
+}
+
+// Path: struct with
+//   SMEM           bytes of dynamic shared memory per block
+//   mark(t)        a triangle begins to die
+//   retire(t)      it died in the round before
+//   debit(g, F, nF, Fn, slot, level, stamp)  the debit phase (all threads call)
+template <class Path>
+__global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path path)
+{
+	uint32_t phase = 0, target = 0, n = 0, mn = 0;
+	uint32_t nF = 0, nPrev = 0, cur = 0, level = 0xffffffffu, round = 0, rounds = 0;
+	const uint64_t tid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+	const uint64_t nthreads = uint64_t(gridDim.x) * blockDim.x;
+	const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+	unsigned long long peeled = 0, ksum = 0, t_start = 0, t_last = 0, ns[4] = {0, 0, 0, 0};
+	if (lead)
+		t_start = t_last = loop_ns();
+	auto lap = [&](int kind) {
+		if (lead)
+		{
+			const unsigned long long now = loop_ns();
+			ns[kind] += now - t_last;
+			t_last = now;
+			if (now - t_start > LOOP_TIME_LIMIT_NS)
+				atomicExch(&g.ctl->abort, 1u);
+		}
+	};
+	bool ok = true;
+	while (peeled < g.T)
+	{
+		uint32_t *F = cur ? g.F1 : g.F0, *Fp = cur ? g.F0 : g.F1;
+		if (nF == 0)
+		{
+			// level change: level + 1 first, else the minimum of the rest
+			scan_level(g, level + 1, F, &g.ctl->slot[phase & 3]);
+			if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+				break;
+			++level;
+			if (lead)
+				g.ctl->scans++;
+			if (n == 0)
+			{
+				if (mn == NO_SUPPORT)
+					break; // nothing alive (cannot happen while peeled < T)
+				level = mn;
+				scan_level(g, level, F, &g.ctl->slot[phase & 3]);
+				if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+					break;
+			}
+			nF = n;
+			lap(2);
+		}
+		const uint32_t stamp = 0x80000000u | round;
+		for (uint64_t i = tid; i < uint64_t(nF) + nPrev; i += nthreads)
+		{
+			if (i < nF)
+			{
+				const uint32_t t = F[i];
+				g.S[t] = int32_t(stamp);
+				g.K[t] = int32_t(level);
+				if (g.R)
+					g.R[t] = round;
+				path.mark(t);
+			}
+			else
+				path.retire(Fp[i - nF]);
+		}
+		if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+			break;
+		lap(0);
+		path.debit(g, F, nF, Fp, &g.ctl->slot[phase & 3], int32_t(level), stamp);
+		if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+			break;
+		lap(1);
+		peeled += nF;
+		ksum += (unsigned long long)level * nF;
+		++rounds;
+		++round;
+		nPrev = nF;
+		nF = n;
+		cur ^= 1u;
+		if (nF >= g.sort_min && nF <= g.T && g.fbits)
+		{
+			order_set(g, Fp, nF);
+			uint32_t unused, m2;
+			if (!(ok = phase_end(g.ctl, phase, target, unused, m2)))
+				break;
+			order_write(g, Fp, &g.ctl->slot[phase & 3]);
+			if (!(ok = phase_end(g.ctl, phase, target, unused, m2)))
+				break;
+			if (lead)
+				g.ctl->ordered++;
+			lap(3);
+		}
+	}
+	if (lead)
+	{
+		PeelCtl &c = g.ctl->c;
+		c.peeled = peeled;
+		c.ksum = ksum;
+		c.kmax = peeled ? level : 0u;
+		c.unpeeled = uint32_t(g.T - peeled);
+		c.rounds = rounds;
+		c.round = round;
+		c.level = level;
+		c.done = ok;
+		for (int i = 0; i < 4; ++i)
+			g.ctl->ns[i] = ns[i];
+		if (!ok)
+			g.ctl->timed_out = 1;
+	}
+}
+
+// Runs the loop on the context's stream and waits for it (peel_loop.cu holds
+// the rest of the host side).
+struct LoopBuffers
+{
+	LoopCtl *ctl = nullptr;
+	uint32_t *R = nullptr, *F0 = nullptr, *F1 = nullptr, *fbits = nullptr;
+};
+int loop_alloc(Ctx &c, LoopBuffers &b);
+void loop_release(Ctx &c, LoopBuffers &b);
+int loop_finish(Ctx &c, LoopBuffers &b, PeelCtl *hctl);
+
+template <class Path>
+int run_peel_loop(Ctx &c, LoopBuffers &b, const Path &path, int32_t *S, int32_t *K)
+{
+	int per_sm = 0;
+	if (cudaFuncSetAttribute(k_peel_loop<Path>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Path::SMEM)) !=
+			cudaSuccess ||
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_loop<Path>, LOOP_THREADS, Path::SMEM) !=
+			cudaSuccess ||
+		per_sm < 1)
+		return fail(NUCLEUS34_E_CUDA, "peel loop occupancy");
+	const nucleus34_tune tn = tune_filled(c.tune);
+	LoopArgs g{b.ctl, S, K, b.R, b.F0, b.F1, b.fbits, c.T, 0xffffffffu};
+	if (tn.sort_shift != NUCLEUS34_TUNE_NEVER)
+		g.sort_min = uint32_t(std::max<uint64_t>(c.T >> tn.sort_shift, 4096));
+	// as many blocks as fit at once, fewer when the scans would leave most of
+	// them without a support word (a barrier costs more the more blocks take part)
+	uint64_t blocks = (c.T + LOOP_THREADS * 4 - 1) / (LOOP_THREADS * 4);
+	blocks = std::min<uint64_t>(std::max<uint64_t>(blocks, 4), uint64_t(per_sm) * uint64_t(c.sm_count));
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(uint32_t(blocks));
+	cfg.blockDim = dim3(LOOP_THREADS);
+	cfg.dynamicSmemBytes = Path::SMEM;
+	cfg.stream = c.stream;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeCooperative;
+	at[0].val.cooperative = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	if (cudaLaunchKernelEx(&cfg, k_peel_loop<Path>, g, path) != cudaSuccess)
+		return fail(NUCLEUS34_E_CUDA, std::string("peel loop: ") + cudaGetErrorString(cudaGetLastError()));
+	c.launches++;
+	return NUCLEUS34_OK;
+}
+
+} // namespace n34

@@ -28,6 +28,23 @@ constexpr uint32_t INC_DEAD = 0x80000000u;
 // round-stamp peel runs. Union passes (batched form, serving) are cut below it.
 constexpr uint64_t FLAG_PEEL_MAX_TRIANGLES = 0x3fffffffull;
 
+// The triangle listing's bit matrices, kept for the on-demand variant. Source
+// u of out-degree d has a d x d matrix of W = ceil(d / 32) cells per row. Row
+// ia belongs to edge O[u] + ia, so an edge stands for its row.
+struct BitMats
+{
+	// x, y: bit ib of row ia is the triangle with head edge a = O[u] + ia and
+	// tail edge b = O[u] + ib; its id is y + the set bits of x below it.
+	// z: symmetric (bit i of row j and bit j of row i are the triangle of u
+	// with the vertices at i and j); the peel clears both when it is dead.
+	// w: symmetric, zero at first; the peel sets both when it begins to die.
+	// One 16-byte load tells a triangle's id and state.
+	uint4 *cells = nullptr;
+	// per oriented edge: {first cell of its row, W << 16 | its position in N+(u)}
+	uint2 *erec = nullptr;
+	uint64_t nwords = 0;
+};
+
 // Triangle -> four-clique incidence of the direct variant.
 struct CliqueCsr
 {
@@ -41,10 +58,14 @@ cudaError_t launch_tri_count(const uint32_t *O, const uint32_t *E, uint64_t n, u
 							 cudaStream_t s);
 cudaError_t launch_tri_write(const uint32_t *O, const uint32_t *E, uint64_t n, const uint64_t *toff,
 							 uint32_t *tris, int sm_count, cudaStream_t s);
-int list_triangles(Ctx &c);
+int list_triangles(Ctx &c, BitMats *keep);
+void free_mats(Ctx &c, BitMats &mats);
 // lean: no 64-bit key array (entries sorted in place as pairs) and no tpos.
 int build_incidence(Ctx &c, Incidence &inc, bool want_tpos, bool lean = false);
 void free_incidence(Ctx &c, Incidence &inc);
+// The in-lists of the bit-matrix form: only the entry under each triangle's c
+// edge (third = its source), so T entries; inc.span/third/tri as above.
+int build_in_lists(Ctx &c, const BitMats &mats, Incidence &inc);
 // Sorts every segment [off[s], off[s+1]) of keys ascending (incidence.cu's
 // segmented sort; nseg < 2^32).
 int sort_segments_u64(Ctx &c, unsigned long long *keys, const uint64_t *off, uint64_t nseg);
@@ -63,6 +84,11 @@ void free_clique_csr(Ctx &c, CliqueCsr &csr);
 int segments_after_listing(Ctx &c);
 int segments_after_support(Ctx &c, const int32_t *support);
 int segments_after_peel(Ctx &c);
+// The bit-matrix form of the support count and the peel (on-demand variant).
+bool bit_form_wanted(const Ctx &c, int variant);
+bool bit_form_fits(const Ctx &c, const BitMats &mats);
+int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, uint64_t *total);
+int peel_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, int32_t *K, PeelCtl *hctl);
 // Device-resident peel; K receives the final k of every triangle.
 int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_t *support, int32_t *K,
 		 PeelCtl *hctl);

@@ -18,12 +18,16 @@
 //               words with 32 ballots into row words M[ia][32q .. 32q+31], and
 //               stores beside each row word the number of set bits before it
 //               in the row; the row totals are the triangles per edge a.
-//   3. offsets  scan of the per-edge-a counts: where each a's triangles start.
+//   3. offsets  scan of the per-edge-a counts: where each a's triangles start;
+//               added to the row prefixes, so that a row word and its prefix
+//               (8 bytes) give the canonical id of each of its triangles.
 //   4. write    the merges of step 1 run again; a common w at A position ia
 //               and B position pb is triangle (O[u]+ia, b, O[v]+pb), and its
-//               canonical position is offset(a) + the row prefix + the set
-//               bits of its row word below ib. No search is needed for c.
-// Steps 1-2 hold 3 words of bits per (column, row tile) of each source; when
+//               canonical position is the row word's first id + the set bits
+//               of the word below ib. No search is needed for c.
+// The matrices can be kept (BitMats) for the on-demand variant's support count
+// and peel (bitpeel.cu).
+// Steps 1-2 hold 20 bytes per (column, row tile) of each source; when
 // those do not fit the budget the sources are taken in chunks, counting all
 // of them first and repeating steps 1-2 before each chunk's writes.
 //
@@ -279,8 +283,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_cols(const uint32_t *__res
 __global__ void __launch_bounds__(TRI_THREADS) k_list_rows(const uint32_t *__restrict__ O, uint64_t u0, uint64_t u1,
 														   const uint64_t *__restrict__ woff, uint64_t wbase,
 														   const uint32_t *__restrict__ cols,
-														   uint32_t *__restrict__ rows, uint32_t *__restrict__ pre,
-														   uint32_t *__restrict__ rowcnt)
+														   uint4 *__restrict__ cells, uint32_t *__restrict__ rowcnt)
 {
 	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 	const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
@@ -309,15 +312,44 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_rows(const uint32_t *__res
 						rw = b;
 				}
 				if (row < d)
-				{
-					rows[base + uint64_t(row) * W + q] = rw;
-					pre[base + uint64_t(row) * W + q] = tot;
-				}
+					cells[base + uint64_t(row) * W + q] = make_uint4(rw, tot, 0u, 0u);
 				tot += __popc(rw);
 			}
 			if (row < d)
 				rowcnt[ob + row] = tot;
 		}
+	}
+}
+
+// Step 3: canonical ids in the cells. One thread per edge a in [j0, j1): the
+// prefix of each of its words becomes the id of the word's first triangle
+// (T < 2^32 was checked). With erec, the column word beside it makes the cell's
+// symmetric word (triangles of u that hold vertex ia and vertex 32q + i,
+// whichever of the two is the head), and the edge's record gets its row and its
+// position.
+__global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__restrict__ O,
+														  const uint32_t *__restrict__ src, uint64_t j0, uint64_t j1,
+														  const uint64_t *__restrict__ woff, uint64_t wbase,
+														  const uint64_t *__restrict__ aoff, uint4 *__restrict__ cells,
+														  const uint32_t *__restrict__ cols, uint2 *__restrict__ erec)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t j = j0 + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < j1; j += stride)
+	{
+		const uint32_t u = __ldg(src + j), ob = __ldg(O + u), d = __ldg(O + u + 1) - ob;
+		const uint32_t W = (d + 31) >> 5, ia = uint32_t(j - ob);
+		const uint64_t base = woff[u] - wbase + uint64_t(ia) * W;
+		const uint32_t first = uint32_t(aoff[j]);
+		for (uint32_t q = 0; q < W; ++q)
+		{
+			uint4 c = cells[base + q];
+			c.y += first;
+			if (erec)
+				c.z = c.x | __ldg(cols + base + q);
+			cells[base + q] = c;
+		}
+		if (erec)
+			erec[j] = make_uint2(uint32_t(base), (W << 16) | ia);
 	}
 }
 
@@ -327,9 +359,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_write(const uint32_t *__re
 															const uint32_t *__restrict__ E,
 															const uint32_t *__restrict__ src, uint64_t j0,
 															uint64_t j1, const uint64_t *__restrict__ woff,
-															uint64_t wbase, const uint32_t *__restrict__ rows,
-															const uint32_t *__restrict__ pre,
-															const uint64_t *__restrict__ aoff, uint64_t T,
+															uint64_t wbase, const uint4 *__restrict__ cells, uint64_t T,
 															uint32_t *__restrict__ tris, uint32_t *__restrict__ err)
 {
 	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -345,8 +375,8 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_write(const uint32_t *__re
 			if (!found)
 				return;
 			const uint32_t ia = (k << 5) + lane_id();
-			const uint64_t at = base + uint64_t(ia) * W + q;
-			const uint64_t pos = aoff[ob + ia] + pre[at] + __popc(rows[at] & below);
+			const uint2 r = __ldg(reinterpret_cast<const uint2 *>(cells + base + uint64_t(ia) * W + q));
+			const uint64_t pos = uint64_t(r.y) + __popc(r.x & below);
 			if (pos < T)
 			{
 				tris[3 * pos + 0] = ob + ia;
@@ -389,15 +419,27 @@ cudaError_t launch_tri_write(const uint32_t *O, const uint32_t *E, uint64_t n, c
 	return cudaGetLastError();
 }
 
-// Lists the triangles of the resident graph into c.dtris (3*T u32) and sets c.T.
-int list_triangles(Ctx &c)
+void free_mats(Ctx &c, BitMats &mats)
+{
+	c.release(mats.cells);
+	c.release(mats.erec);
+	mats = BitMats{};
+}
+
+// Lists the triangles of the resident graph into c.dtris (3*T u32) and sets
+// c.T. With keep, the bit matrices stay behind in *keep when they were built in
+// one chunk and their positions fit the edge records (32-bit word positions,
+// 16-bit row positions); else *keep is left empty.
+int list_triangles(Ctx &c, BitMats *keep)
 {
 	c.T = 0;
 	if (c.m == 0)
 		return NUCLEUS34_OK;
 	const uint64_t n = c.n, m = c.m;
 	uint64_t *words = nullptr, *woff = nullptr, *aoff = nullptr;
-	uint32_t *rowcnt = nullptr, *cols = nullptr, *rows = nullptr, *pre = nullptr, *err = nullptr;
+	uint32_t *rowcnt = nullptr, *cols = nullptr, *err = nullptr;
+	uint4 *cells = nullptr;
+	uint2 *erec = nullptr;
 	int rc = NUCLEUS34_OK;
 	auto cleanup = [&] {
 		c.release(words);
@@ -405,8 +447,8 @@ int list_triangles(Ctx &c)
 		c.release(aoff);
 		c.release(rowcnt);
 		c.release(cols);
-		c.release(rows);
-		c.release(pre);
+		c.release(cells);
+		c.release(erec);
 		c.release(err);
 	};
 	do
@@ -434,10 +476,10 @@ int list_triangles(Ctx &c)
 		words = nullptr;
 		if ((rc = dalloc(c, &rowcnt, m, "triangles per edge")) || (rc = dalloc(c, &aoff, m + 1, "triangle offsets")))
 			break;
-		// Chunks of sources whose bit words (3 arrays) fit a quarter of the
-		// room left; one chunk when all of them do.
+		// Chunks of sources whose words (a column word and a cell) fit a
+		// quarter of the room left; one chunk when all of them do.
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
-		uint64_t cap_words = std::max<uint64_t>(room / 4 / 12, uint64_t(1) << 20);
+		uint64_t cap_words = std::max<uint64_t>(room / 4 / 20, uint64_t(1) << 20);
 		// NUCLEUS34_LIST_CHUNK_WORDS=N caps the chunk at N words (a test hook
 		// for the chunked path, which budgets alone reach only on large graphs)
 		if (const char *e = std::getenv("NUCLEUS34_LIST_CHUNK_WORDS"))
@@ -495,8 +537,7 @@ int list_triangles(Ctx &c)
 			maxw = std::max(maxw, hwc[i + 1] - hwc[i]);
 		const uint64_t alloc_w = maxw ? maxw : 1;
 		if ((rc = dalloc(c, &cols, alloc_w, "listing column words")) ||
-			(rc = dalloc(c, &rows, alloc_w, "listing row words")) ||
-			(rc = dalloc(c, &pre, alloc_w, "listing row prefixes")))
+			(rc = dalloc(c, &cells, alloc_w, "listing cells")))
 			break;
 		const size_t nchunks = cuts.size() - 1;
 		auto bits_of_chunk = [&](size_t i) -> int {
@@ -505,7 +546,7 @@ int list_triangles(Ctx &c)
 				N34_LAUNCH(c, k_list_cols, grid_for(c, j1 - j0, TRI_WARPS, 32), TRI_THREADS, 0, c.dO, c.dE, c.dsrc,
 						   j0, j1, woff, hwc[i], cols);
 			N34_LAUNCH(c, k_list_rows, grid_for(c, u1 - u0, TRI_WARPS, 32), TRI_THREADS, 0, c.dO, u0, u1, woff,
-					   hwc[i], cols, rows, pre, rowcnt);
+					   hwc[i], cols, cells, rowcnt);
 			return NUCLEUS34_OK;
 		};
 		// counts of every chunk, then the offsets
@@ -528,8 +569,20 @@ int list_triangles(Ctx &c)
 		c.T = T;
 		if (T == 0)
 			break;
+		if (nchunks == 1)
+		{
+			c.release(rowcnt);
+			rowcnt = nullptr;
+		}
 		if ((rc = dalloc(c, &c.dtris, 3 * T, "triangles")))
 			break;
+		bool kept = keep && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu;
+		if (kept && dalloc(c, &erec, m, "edge records"))
+		{
+			erec = nullptr; // the matrices are not kept then
+			kept = false;
+			clear_error();
+		}
 		for (size_t i = 0; i < nchunks && !rc; ++i)
 		{
 			// a single chunk still holds its bits from the count
@@ -538,9 +591,11 @@ int list_triangles(Ctx &c)
 			const uint64_t j0 = hO[i], j1 = hO[i + 1];
 			if (j1 > j0)
 			{
+				k_list_ids<<<grid_for(c, j1 - j0, TRI_THREADS, 32), TRI_THREADS, 0, c.stream>>>(
+					c.dO, c.dsrc, j0, j1, woff, hwc[i], aoff, cells, cols, erec);
 				k_list_write<<<grid_for(c, j1 - j0, TRI_WARPS, 32), TRI_THREADS, 0, c.stream>>>(
-					c.dO, c.dE, c.dsrc, j0, j1, woff, hwc[i], rows, pre, aoff, T, c.dtris, err);
-				c.launches++;
+					c.dO, c.dE, c.dsrc, j0, j1, woff, hwc[i], cells, T, c.dtris, err);
+				c.launches += 2;
 			}
 		}
 		if (rc)
@@ -554,6 +609,12 @@ int list_triangles(Ctx &c)
 		}
 		if (herr)
 			rc = fail(NUCLEUS34_E_CUDA, "internal: triangle listing check failed");
+		else if (kept)
+		{
+			*keep = BitMats{cells, erec, nwords};
+			cells = nullptr;
+			erec = nullptr;
+		}
 	} while (false);
 	cleanup();
 	return rc;
