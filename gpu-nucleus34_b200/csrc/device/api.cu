@@ -413,7 +413,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 			// k is kept in the support array and becomes the result
 			if (total)
 			{
-				if ((rc = peel(c, variant, inc, csr, S, S, &pc)))
+				if ((rc = peel(c, inc, S, S, &pc)))
 					break;
 				peeled = true;
 			}
@@ -430,7 +430,10 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (total)
 			{
-				if ((rc = bits ? peel_bits(c, mats, inc, S, c.dK, &pc) : peel(c, variant, inc, csr, S, c.dK, &pc)))
+				rc = variant == NUCLEUS34_DIRECT ? peel_direct(c, csr, S, c.dK, &pc)
+					 : bits						 ? peel_bits(c, mats, inc, S, c.dK, &pc)
+												 : peel(c, inc, S, c.dK, &pc);
+				if (rc)
 					break;
 				peeled = true;
 			}

@@ -345,22 +345,7 @@ struct BitPath
 			}
 			const uint32_t id[3] = {id1, id2, id3};
 			const bool live[3] = {live1, live2, live3};
-			int32_t old[3];
-#pragma unroll
-			for (int k = 0; k < 3; ++k)
-			{
-				old[k] = 0x7fffffff;
-				if (ok && live[k])
-					old[k] = atomicSub(S + id[k], 1);
-			}
-			const bool hit = old[0] == level + 1 || old[1] == level + 1 || old[2] == level + 1;
-			if (__any_sync(FULL, hit))
-			{
-#pragma unroll
-				for (int k = 0; k < 3; ++k)
-					next.push(old[k] == level + 1, id[k]);
-				next.drain();
-			}
+			next.debit(ok, id, live, S, level);
 			queued = 0;
 			__syncwarp();
 		}

@@ -1,8 +1,8 @@
-// Device-resident, level-synchronous bucketed peel of triangle support.
+// Device-resident, level-synchronous bucketed peel of triangle support on the
+// incidence lists: the on-demand variant's list form, for graphs whose bit
+// matrices do not fit (bitpeel.cu) and for the flags that ask for it.
 //
-// Reference: the direct program launches peel_fourcliques over ALL triangles
-// once per level with a host round trip each (nucleus/cuNucleus34.cu:107-141,
-// 675-714; claim flags per clique), the on-demand program runs
+// Reference: the on-demand program runs
 // min_alive_support / mark_dying / debit_partners with three device->host
 // copies and two syncs per round (cuNucleus34_ondemand.cu:203-305, 599-682);
 // the CPU form is bucket_ex::peeling_par (nucleus/bucket_ex.hpp:274-360).
@@ -14,14 +14,14 @@
 //   scan_min / gather  (only when the frontier is empty): next level = min
 //                      alive support; frontier = alive triangles at it.
 //   mark               K[t] = level, R[t] = round for the frontier.
-//   debit              each dying triangle enumerates its cliques (on-demand:
-//                      3-way intersection of its incidence lists; direct: its
-//                      clique ids); the clique belongs to its first member to
-//                      die, ties to the lowest id (the death-stamp rule of
-//                      debit_partners, cuNucleus34_ondemand.cu:237-276); the
-//                      owner debits every alive partner with atomicSub. A
-//                      partner whose support falls from level+1 to level is
-//                      appended to the next frontier (exactly once).
+//   debit              each dying triangle enumerates its cliques (3-way
+//                      intersection of its incidence lists); the clique
+//                      belongs to its first member to die, ties to the lowest
+//                      id (the death-stamp rule of debit_partners,
+//                      cuNucleus34_ondemand.cu:237-276); the owner debits every
+//                      alive partner with atomicSub. A partner whose support
+//                      falls from level+1 to level is appended to the next
+//                      frontier (exactly once).
 //   advance            swap frontiers, advance the round.
 // The result is independent of thread timing: ownership depends only on the
 // stamps, and crossing detection catches every triangle that reaches the level.
@@ -490,94 +490,6 @@ __global__ void __launch_bounds__(PEEL_THREADS) k_debit_ondemand(
 			}
 			settle_clique(found, t, q0, q1, q2, K, R, S, round, level, Fn, &ctl->c.nNext, T, &ctl->c.error);
 		});
-	}
-}
-
-// Direct variant: a dying triangle walks its clique ids. A clique destroyed in
-// an earlier round carries a set byte in `destroyed` (written by its owner), so
-// later members skip it with one byte load; otherwise the members are read and
-// the round-stamp owner rule decides.
-__global__ void __launch_bounds__(PEEL_THREADS) k_debit_direct(
-	CtlX *ctl, uint32_t *__restrict__ F0, uint32_t *__restrict__ F1, const uint64_t *__restrict__ coff,
-	const uint32_t *__restrict__ cids, const uint4 *__restrict__ quds, const int32_t *__restrict__ K,
-	const uint32_t *__restrict__ R, int32_t *__restrict__ S, uint8_t *__restrict__ destroyed, uint64_t T)
-{
-	if (ctl->c.done)
-		return;
-	const uint32_t nF = ctl->c.nF;
-	const uint32_t *F = ctl->c.cur ? F1 : F0;
-	uint32_t *Fn = ctl->c.cur ? F0 : F1;
-	const int32_t level = int32_t(ctl->c.level);
-	const uint32_t round = ctl->c.round;
-	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-	for (uint64_t i = warp; i < nF; i += nwarps)
-	{
-		const uint32_t t = F[i];
-		const uint64_t b = coff[t], e = coff[t + 1];
-		for (uint64_t base = b; base < e; base += 32)
-		{
-			const uint64_t j = base + lane_id();
-			bool live = false;
-			uint32_t q = 0, q0 = 0, q1 = 0, q2 = 0;
-			if (j < e)
-			{
-				q = cids[j];
-				live = !destroyed[q];
-			}
-			if (live)
-			{
-				const uint4 x = quds[q];
-				// the three members other than t
-				const uint32_t m[4] = {x.x, x.y, x.z, x.w};
-				uint32_t o[3] = {0, 0, 0};
-				int k = 0;
-#pragma unroll
-				for (int s = 0; s < 4; ++s)
-					if (m[s] != t && k < 3)
-						o[k++] = m[s];
-				q0 = o[0];
-				q1 = o[1];
-				q2 = o[2];
-			}
-			bool owner = live;
-			bool al[3] = {false, false, false};
-			if (live)
-			{
-				const uint32_t p[3] = {q0, q1, q2};
-#pragma unroll
-				for (int s = 0; s < 3; ++s)
-				{
-					al[s] = K[p[s]] == -1;
-					if (!al[s] && (R[p[s]] < round || p[s] < t))
-						owner = false;
-				}
-			}
-			bool hit[3] = {false, false, false};
-			if (owner)
-			{
-				destroyed[q] = 1;
-				if (al[0])
-					hit[0] = atomicSub(S + q0, 1) == level + 1;
-				if (al[1])
-					hit[1] = atomicSub(S + q1, 1) == level + 1;
-				if (al[2])
-					hit[2] = atomicSub(S + q2, 1) == level + 1;
-			}
-			const uint32_t qs[3] = {q0, q1, q2};
-#pragma unroll
-			for (int r = 0; r < 3; ++r)
-			{
-				const uint32_t slot = warp_append(hit[r], &ctl->c.nNext);
-				if (hit[r])
-				{
-					if (slot < T)
-						Fn[slot] = qs[r];
-					else
-						atomicOr(&ctl->c.error, 1u);
-				}
-			}
-		}
 	}
 }
 
@@ -1796,12 +1708,11 @@ uint32_t small_rounds_grid(int sm_count)
 
 } // namespace
 
-int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_t *S, int32_t *K, PeelCtl *hctl)
+int peel(Ctx &c, const Incidence &inc, int32_t *S, int32_t *K, PeelCtl *hctl)
 {
 	const uint64_t T = c.T;
 	uint32_t *R = nullptr, *F0 = nullptr, *F1 = nullptr, *B0 = nullptr, *B1 = nullptr, *fbits = nullptr,
 			 *fchunk = nullptr;
-	uint8_t *destroyed = nullptr;
 	CtlX *ctl = nullptr;
 	GridBar *bar = nullptr;
 	int rc = NUCLEUS34_OK;
@@ -1815,11 +1726,10 @@ int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_
 		c.release(fchunk);
 		c.release(ctl);
 		c.release(bar);
-		c.release(destroyed);
 	};
 	// death flags live in the incidence entries when triangle ids leave the
 	// top two bits free (the incidence is discarded after the peel)
-	const bool flags = variant == NUCLEUS34_ONDEMAND && T <= ID_MASK && !(c.opt_flags & NUCLEUS34_OPT_STAMP_PEEL);
+	const bool flags = T <= ID_MASK && !(c.opt_flags & NUCLEUS34_OPT_STAMP_PEEL);
 	// death rounds: the round-stamp owner test needs them; the death-flag
 	// path records them only to keep them for nucleus34_ctx_verify
 	const bool keep_rounds = (c.opt_flags & NUCLEUS34_OPT_VERIFIABLE) != 0;
@@ -1928,16 +1838,6 @@ int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_
 			break;
 		}
 		const uint32_t gsort = uint32_t(std::min<uint64_t>(fchunks, uint64_t(c.sm_count) * 8));
-		if (variant == NUCLEUS34_DIRECT)
-		{
-			if ((rc = dalloc(c, &destroyed, c.Q ? c.Q : 1, "clique destroyed flags")))
-				break;
-			if (cudaMemsetAsync(destroyed, 0, c.Q ? c.Q : 1, c.stream) != cudaSuccess)
-			{
-				rc = fail(NUCLEUS34_E_CUDA, "memset");
-				break;
-			}
-		}
 		const uint32_t gscan = grid_for(c, T, PEEL_THREADS, 8);
 		const uint32_t gwarp = grid_for(c, T, PEEL_THREADS / 32, 16);
 		k_peel_init<<<gscan, PEEL_THREADS, 0, c.stream>>>(Kw, T, ctl, compact_div, sort_min);
@@ -2009,13 +1909,8 @@ int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_
 			{
 				k_mark<<<gscan, PEEL_THREADS, 0, c.stream>>>(ctl, F0, F1, K, R, S);
 				tick(4);
-				if (variant == NUCLEUS34_ONDEMAND)
-					k_debit_ondemand<<<gwarp, PEEL_THREADS, 0, c.stream>>>(ctl, F0, F1, c.dtris, inc.span, inc.third,
-																		   inc.tri, K, R, S, T);
-				else
-					k_debit_direct<<<gwarp, PEEL_THREADS, 0, c.stream>>>(
-						ctl, F0, F1, csr.off, csr.ids, reinterpret_cast<const uint4 *>(c.dquds), K, R, S, destroyed,
-						T);
+				k_debit_ondemand<<<gwarp, PEEL_THREADS, 0, c.stream>>>(ctl, F0, F1, c.dtris, inc.span, inc.third, inc.tri,
+																	   K, R, S, T);
 				tick(5);
 				tick(6);
 				tick(7);
@@ -2261,7 +2156,7 @@ int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_
 				std::fprintf(stderr, " %s=%.1fms", prof_names[j], prof_ms[j]);
 			std::fprintf(stderr, "\n");
 			// steps 4 and 5: the debit kernels (thread + warp, or the single
-			// stamp/direct debit in slot 4)
+			// stamp debit in slot 4)
 			c.peel_debit_sec = (prof_ms[4] + prof_ms[5]) * 1e-3;
 		}
 		if (exec)

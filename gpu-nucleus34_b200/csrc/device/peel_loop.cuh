@@ -163,6 +163,26 @@ struct Appender
 			buf[count + __popc(m & lanemask_lt())] = t;
 		count += __popc(m);
 	}
+	// A clique that the lanes with own set destroy: debits its live partners and
+	// collects those that fall to the level (all lanes call).
+	__device__ __forceinline__ void debit(bool own, const uint32_t id[3], const bool live[3], int32_t *S, int32_t level)
+	{
+		// all three in flight before the first result is used
+		int32_t old[3];
+#pragma unroll
+		for (int r = 0; r < 3; ++r)
+		{
+			old[r] = 0x7fffffff;
+			if (own && live[r])
+				old[r] = atomicSub(S + id[r], 1);
+		}
+		if (!__any_sync(FULL, old[0] == level + 1 || old[1] == level + 1 || old[2] == level + 1))
+			return;
+#pragma unroll
+		for (int r = 0; r < 3; ++r)
+			push(old[r] == level + 1, id[r]);
+		drain();
+	}
 	// makes room for three pushes (all lanes call)
 	__device__ __forceinline__ void drain()
 	{

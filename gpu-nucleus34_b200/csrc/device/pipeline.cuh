@@ -89,9 +89,10 @@ bool bit_form_wanted(const Ctx &c, int variant);
 bool bit_form_fits(const Ctx &c, const BitMats &mats);
 int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, uint64_t *total);
 int peel_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, int32_t *K, PeelCtl *hctl);
-// Device-resident peel; K receives the final k of every triangle.
-int peel(Ctx &c, int variant, const Incidence &inc, const CliqueCsr &csr, int32_t *support, int32_t *K,
-		 PeelCtl *hctl);
+// The direct variant's peel over the clique list.
+int peel_direct(Ctx &c, const CliqueCsr &csr, int32_t *support, int32_t *K, PeelCtl *hctl);
+// Device-resident peel of the on-demand variant's list form; K receives the final k of every triangle.
+int peel(Ctx &c, const Incidence &inc, int32_t *support, int32_t *K, PeelCtl *hctl);
 
 // Certificate check of the last run (verify.cu); needs the kept death rounds.
 int verify(Ctx &c, uint64_t *violations, uint64_t *checked);

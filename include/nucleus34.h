@@ -78,17 +78,26 @@ typedef struct
 /* opts.flags: force the round-stamp ownership test in the on-demand peel
  * (the default keeps death flags inside the incidence entries when T < 2^30). */
 #define NUCLEUS34_OPT_STAMP_PEEL 0x1u
-/* opts.flags: run the peel rounds as plain launches with CUDA events around
- * every step and print per-step device times to stderr (diagnostics only;
- * slower than the default graph replay). */
+/* opts.flags: print the peel's device time per step (mark, debit, level scan,
+ * frontier order) to stderr and return the debit's in t_peel_debit. With a
+ * flag below that selects the list form of the on-demand peel, its rounds run
+ * as plain launches with CUDA events around every step (slower). */
 #define NUCLEUS34_OPT_PROFILE_PEEL 0x2u
-/* opts.flags: the memory-lean layout of the on-demand variant (T < 2^30):
+/* The on-demand variant peels on the triangle listing's bit matrices, all
+ * rounds in one cooperative launch, as the direct variant does on its clique
+ * list. Its list form, on the incidence lists, serves graphs whose matrices do
+ * not fit in the memory budget, and the flags below that select a layout or a
+ * schedule of it (STAMP_PEEL, LEAN_MEMORY, HOST_LOOP, NO_SMALL_ROUNDS,
+ * FRONTIER_BY_C, CHUNKED_DEBIT, SCALAR_SCANS, PIPELINED_DEBIT, DEBIT_CURSOR;
+ * they do not concern the direct variant). Results are identical. */
+/* opts.flags: the memory-lean layout of the list form (T < 2^30):
  * incidence entries sorted in place (no 64-bit sort keys beside them), no
  * per-triangle entry positions (the peel searches for a triangle's entries),
  * frontiers as two bitmaps instead of two lists, and k kept in the support
  * array; about 28 bytes per triangle beside the triangle list instead of
- * about 60. Chosen automatically when the regular layout does not fit in
- * the memory budget left after the triangle listing. Results are identical. */
+ * about 60. Chosen automatically when the list form's regular layout does not
+ * fit in the memory budget left after the triangle listing. Results are
+ * identical. */
 #define NUCLEUS34_OPT_LEAN_MEMORY 0x4u
 /* opts.flags: keep each triangle's death round after the peel, so that
  * nucleus34_ctx_verify can certify the result (costs 4 bytes per triangle). */
