@@ -617,10 +617,9 @@ int nucleus34_batch_copy_k(nucleus34_batch b, uint64_t index, int32_t *k_out, ui
 		}
 		N34_CUDA(cudaSetDevice(c.device));
 		if (k_out)
-			N34_CUDA(cudaMemcpyAsync(k_out, c.dK + t0, T * 4, cudaMemcpyDeviceToHost, c.stream));
+			N34_TRY(copy_to_host(c, k_out, c.dK + t0, T * 4));
 		if (tris_out)
-			N34_CUDA(cudaMemcpyAsync(tris_out, c.dtris + 3 * t0, T * 12, cudaMemcpyDeviceToHost, c.stream));
-		N34_CUDA(cudaStreamSynchronize(c.stream));
+			N34_TRY(copy_to_host(c, tris_out, c.dtris + 3 * t0, T * 12));
 		if (tris_out)
 		{
 			// edge ids of the graph alone

@@ -99,6 +99,7 @@ int verify(Ctx &c, uint64_t *violations, uint64_t *checked);
 // Context entry points shared by the C-ABI front ends (api.cu, batch.cu).
 int upload(Ctx &c, const nucleus34_csr *csr);
 int run(Ctx &c, int variant, nucleus34_result *out);
+int copy_to_host(Ctx &c, void *dst, const void *src, uint64_t bytes);
 int create_ctx(const nucleus34_opts *opts, nucleus34_ctx *out);
 void destroy_ctx(nucleus34_ctx x);
 

@@ -208,7 +208,8 @@ int nucleus34_write_kfile(nucleus34_handle h, const char *path);
 void nucleus34_free(nucleus34_handle h);
 
 /* Returns the device memory cached by earlier calls (the default memory pool
- * of `device`, trimmed to zero) to the driver. */
+ * of `device`, trimmed to zero) to the driver, and frees the process's idle
+ * pinned buffers for result copies. */
 int nucleus34_release_cached_memory(int device);
 
 const char *nucleus34_strerror(int code);
