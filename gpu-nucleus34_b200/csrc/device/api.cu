@@ -486,7 +486,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 // shared by the contexts of the process: a copy borrows a set for its duration.
 // At most STAGE_SETS idle sets are kept (32 MB each; making one takes about
 // 13 ms); nucleus34_release_cached_memory frees them.
-constexpr uint64_t COPY_STAGED = 8ull << 20, COPY_CHUNK = 16ull << 20, COPY_PART = 2ull << 20;
+constexpr uint64_t COPY_STAGED = 20ull << 20, COPY_CHUNK = 16ull << 20, COPY_PART = 2ull << 20;
 constexpr size_t STAGE_BUFFERS = 2, STAGE_SETS = 2;
 static std::mutex stage_mu;
 static std::vector<void *> stage_idle;
@@ -537,8 +537,8 @@ static void free_stages()
 // threads move each chunk on: the runtime's own copy to memory that the caller
 // has just allocated runs at 4.8 GB/s, as one thread takes the destination's
 // page faults (448 MB of k: 94 ms); this one at 25 GB/s (18 ms; with chunks of
-// 8 MB 27 ms, with parts that share huge pages 50 ms). From 8 MB on: below, the
-// runtime's copy takes 1 to 2 ms and the threads gain little.
+// 8 MB 27 ms, with parts that share huge pages 50 ms). From 20 MB on: 11 MB take
+// the runtime's copy 1.5 ms and this one up to 2.4, 62 MB 13.8 and 2.7.
 int copy_to_host(Ctx &c, void *dst, const void *src, uint64_t bytes)
 {
 	cudaPointerAttributes at{};

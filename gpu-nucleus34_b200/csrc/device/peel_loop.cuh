@@ -17,7 +17,8 @@
 // Round-to-round cost is what bounds the small graphs and the long tails of
 // the large ones: with every step of a round a kernel of its own (13 launches
 // in a CUDA graph's while node) a round took 38 us on R-MAT scale 12 and 66 us
-// on scale 16, with most of the launches empty; here it takes 14 and 40 us.
+// on scale 16, with most of the launches empty; here it takes 13 and 33 us, of
+// which a barrier is 1.4.
 //
 // The counters that a phase fills (appended triangles, minimum support) live
 // in one of four slots taken in turn; every block reads the slot right after
@@ -42,19 +43,18 @@ constexpr uint32_t NO_SUPPORT = 0xffffffffu;
 constexpr unsigned long long LOOP_WAIT_LIMIT_NS = 60ull * 1000000000ull;
 constexpr unsigned long long LOOP_TIME_LIMIT_NS = 600ull * 1000000000ull;
 
-struct PhaseSlot
+struct alignas(16) PhaseSlot
 {
-	uint32_t n;    // triangles appended in the phase
-	uint32_t mn;   // least support above the gathered level (scan phase)
-	uint32_t work; // units of the debit phase claimed beyond the first of each warp
-	uint32_t pad;
+	uint32_t arrived; // blocks at the phase's barrier
+	uint32_t n;       // triangles appended in the phase (read with arrived, in one 64-bit load)
+	uint32_t mn;      // least support above the gathered level (scan phase)
+	uint32_t work;    // units of the debit phase claimed beyond the first of each warp
 };
 
 struct LoopCtl
 {
 	PeelCtl c; // results: peeled, ksum, kmax, rounds, error
 	uint32_t timed_out;
-	uint32_t arrived; // barrier arrivals, never reset (compared modulo 2^32)
 	uint32_t abort;
 	uint32_t scans, ordered;
 	PhaseSlot slot[4];
@@ -73,18 +73,28 @@ struct LoopArgs
 	uint32_t sort_min; // frontiers at least this large are put in id order
 };
 
+// A warp's number in the launch: the first warps of all blocks, then their
+// second warps, and so on, so that few warps' work is on as many SMs.
+__device__ __forceinline__ uint32_t loop_warp() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ uint32_t loop_warps() { return (gridDim.x * blockDim.x) >> 5; }
+
+// f(i) for i in [0, n): every block takes an equal, contiguous share (whole
+// warps), so that a small n is spread over all SMs and a large one keeps
+// neighbours on one SM.
+template <class Fn>
+__device__ __forceinline__ void block_shares(uint64_t n, Fn &&f)
+{
+	const uint64_t share = ((n + gridDim.x - 1) / gridDim.x + 31) & ~uint64_t(31);
+	const uint64_t end = min(n, (blockIdx.x + 1) * share);
+	for (uint64_t i = blockIdx.x * share + threadIdx.x; i < end; i += blockDim.x)
+		f(i);
+}
+
 __device__ __forceinline__ unsigned long long loop_ns()
 {
 	unsigned long long t;
 	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
 	return t;
-}
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
-{
-	uint32_t v;
-	asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-	return v;
 }
 
 // A support word: weak load. Its sign and stamp only change in the mark phase;
@@ -238,11 +248,10 @@ __device__ __forceinline__ bool partner_blocks(int32_t s, uint32_t id, uint32_t 
 	return s < 0 && (uint32_t(s) != stamp || id < t);
 }
 
-// How a debit phase is cut into units, which the warps claim as they go (the
-// first by their number, the others from the slot's counter): batches of ch
-// consecutive frontier triangles, at least sixteen per warp (a fixed stride
-// over two per warp took 325 ms of debit on R-MAT scale 18, claimed units of
-// that size 247); or, where the frontier has at most half as many triangles as
+// How a debit phase is cut into units, which are claimed as the warps go:
+// batches of ch consecutive frontier triangles, at least sixteen per warp (a
+// fixed stride over two per warp took 325 ms of debit on R-MAT scale 18,
+// claimed units of that size 247); or, where the frontier has at most half as many triangles as
 // there are warps, one triangle shared by 2^shift warps (twice or four times as
 // many warps per triangle: 17% and 35% slower on R-MAT scale 12).
 struct Units
@@ -262,45 +271,103 @@ __device__ __forceinline__ Units debit_units(uint32_t nF, uint32_t nwarps)
 	return u;
 }
 
-// f(unit) for every unit of the phase (all lanes call f together).
+// f(unit) for every unit of the phase (all lanes call f together; all threads
+// of the block call). A block claims `grab` consecutive units at a time and its
+// warps take them one by one, so that the warps of an SM work on neighbouring
+// triangles, whose rows and supports are in the same lines and pages: against
+// claims by single warps the peel takes 175 ms instead of 250 on R-MAT scale
+// 18, 36 instead of 44 on scale 16, 56 instead of 62 on the geometric graph
+// with 500k points (address translation limits scattered accesses: 1.3e5 lines
+// that stay in L2 are read 2.7e11 times a second from 128 MB of addresses, 5.3e10
+// from 512 MB; up to 256 units per claim make no difference).
 template <class Fn>
 __device__ __forceinline__ void claim_units(uint32_t total, uint32_t *work, Fn &&f)
 {
-	const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-	const uint32_t grab = min(max(total / (nwarps * 8), 1u), 16u); // units per claim
-	for (uint32_t unit = warp * grab; unit < total;)
+	const uint32_t nwarps = loop_warps();
+	if (total <= nwarps)
 	{
-		uint32_t next = total;
-		if (total > nwarps * grab && lane_id() == 0)
-			next = nwarps * grab + atomicAdd(work, grab); // its latency is hidden by f
-		const uint32_t end = min(unit + grab, total);
-		for (; unit < end; ++unit)
-			f(unit);
-		unit = __shfl_sync(FULL, next, 0);
+		// one unit each, on as many SMs as there are units
+		if (loop_warp() < total)
+			f(loop_warp());
+		return;
+	}
+	// high word: end of the claimed range, low word: its next unit
+	__shared__ unsigned long long s_range;
+	const uint32_t grab = min(max(total / (gridDim.x * 8), 1u), 16u);
+	if (threadIdx.x == 0)
+	{
+		const uint32_t b = blockIdx.x * grab;
+		s_range = b < total ? (unsigned long long)min(b + grab, total) << 32 | b : (unsigned long long)total << 32 | total;
+	}
+	__syncthreads();
+	for (;;)
+	{
+		uint32_t unit = total;
+		if (lane_id() == 0)
+		{
+			for (;;)
+			{
+				const unsigned long long r = atomicAdd(&s_range, 1ull);
+				const uint32_t at = uint32_t(r), end = uint32_t(r >> 32);
+				if (at < end)
+				{
+					unit = at;
+					break;
+				}
+				if (end == total)
+					break; // nothing lies past it
+				if (at == end)
+				{
+					// this warp fetches the next range
+					const uint32_t b = gridDim.x * grab + atomicAdd(work, grab);
+					if (b >= total)
+					{
+						atomicExch(&s_range, (unsigned long long)total << 32 | total);
+						break;
+					}
+					atomicExch(&s_range, (unsigned long long)min(b + grab, total) << 32 | (b + 1));
+					unit = b;
+					break;
+				}
+				// another warp is fetching it
+				while ((uint32_t)(*(volatile unsigned long long *)&s_range >> 32) == end)
+					__nanosleep(32);
+			}
+		}
+		unit = __shfl_sync(FULL, unit, 0);
+		if (unit >= total)
+			break;
+		f(unit);
 	}
 }
 
-// End of a phase: grid barrier, then the phase's slot. False: leave.
-__device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_t &target, uint32_t &n, uint32_t &mn)
+// End of a phase: grid barrier; n gets the phase's appended triangles and mn,
+// with scan set, its least support. False: leave.
+__device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_t &n, uint32_t &mn, bool scan)
 {
 	__shared__ uint32_t s_n, s_mn, s_ok;
 	__syncthreads();
 	if (threadIdx.x == 0)
 	{
+		PhaseSlot *slot = &ctl->slot[phase & 3];
 		if (blockIdx.x == 0)
-			ctl->slot[(phase + 2) & 3] = PhaseSlot{0u, NO_SUPPORT, 0u, 0u};
-		__threadfence();
-		target += gridDim.x;
-		atomicAdd(&ctl->arrived, 1u);
-		uint32_t spins = 0;
-		unsigned long long t0 = 0;
-		while (int32_t(ld_acquire(&ctl->arrived) - target) < 0)
+			ctl->slot[(phase + 2) & 3] = PhaseSlot{0u, 0u, NO_SUPPORT, 0u};
+		// the block's writes before its arrival
+		asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&slot->arrived) : "memory");
+		uint32_t spins = 0, ok = 1;
+		unsigned long long t0 = 0, v;
+		for (;;)
 		{
+			asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(slot) : "memory");
+			if (uint32_t(v) >= gridDim.x)
+				break;
 			if ((++spins & 1023u) == 0)
 			{
 				if (__ldcg(&ctl->abort))
+				{
+					ok = 0;
 					break;
+				}
 				const unsigned long long now = loop_ns();
 				if (!t0)
 					t0 = now;
@@ -308,10 +375,11 @@ __device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_
 					atomicExch(&ctl->abort, 1u);
 			}
 		}
-		__threadfence();
-		s_n = __ldcg(&ctl->slot[phase & 3].n);
-		s_mn = __ldcg(&ctl->slot[phase & 3].mn);
-		s_ok = __ldcg(&ctl->abort) == 0;
+		asm volatile("fence.acq_rel.gpu;" ::: "memory");
+		s_n = uint32_t(v >> 32);
+		if (scan)
+			s_mn = __ldcg(&slot->mn);
+		s_ok = ok;
 	}
 	__syncthreads();
 	++phase;
@@ -321,20 +389,24 @@ __device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_
 }
 
 // Appends every live triangle with support <= hi to F and takes the minimum of
-// the others. A warp reads 1024 supports per step, eight per thread at a time
-// (two 16-byte loads), and appends them with one atomic.
+// the others. A warp reads up to 1024 supports per step, eight per thread at a
+// time (two 16-byte loads), and appends them with one atomic.
 __device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint32_t *__restrict__ F, PhaseSlot *slot)
 {
 	const uint32_t lane = lane_id();
-	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t stride = ((uint64_t(gridDim.x) * blockDim.x) >> 5) * 1024;
+	const uint64_t warp = loop_warp();
+	// 1024 supports a step, 256 where that leaves warps without any
+	const uint32_t chunks = g.T >= uint64_t(loop_warps()) * 1024 ? 4 : 1;
+	const uint64_t stride = uint64_t(loop_warps()) * chunks * 256;
 	uint32_t mn = NO_SUPPORT;
-	for (uint64_t b0 = warp * 1024; b0 < g.T; b0 += stride)
+	for (uint64_t b0 = warp * chunks * 256; b0 < g.T; b0 += stride)
 	{
 		uint32_t mask = 0; // bit 8c + j: support j of this lane's chunk c
 #pragma unroll
 		for (uint32_t c = 0; c < 4; ++c)
 		{
+			if (c >= chunks)
+				break;
 			const uint64_t t0 = b0 + c * 256 + lane * 8;
 			int32_t v[8];
 			if (t0 + 8 <= g.T)
@@ -373,8 +445,7 @@ __device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint3
 		if (lane == 0)
 			base = atomicAdd(&slot->n, total);
 		base = __shfl_sync(FULL, base, 0);
-#pragma unroll
-		for (uint32_t c = 0; c < 4; ++c)
+		for (uint32_t c = 0; c < chunks; ++c)
 		{
 			uint32_t z = (mask >> (c * 8)) & 0xffu;
 			const uint32_t x = warp_incl_scan(__popc(z));
@@ -392,23 +463,29 @@ __device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint3
 			base += __shfl_sync(FULL, x, 31);
 		}
 	}
+	// one atomic per block
+	__shared__ uint32_t s_min;
+	if (threadIdx.x == 0)
+		s_min = NO_SUPPORT;
+	__syncthreads();
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1)
 		mn = min(mn, __shfl_xor_sync(FULL, mn, o));
 	if (lane == 0 && mn != NO_SUPPORT)
-		atomicMin(&slot->mn, mn);
+		atomicMin(&s_min, mn);
+	__syncthreads();
+	if (threadIdx.x == 0 && s_min != NO_SUPPORT)
+		atomicMin(&slot->mn, s_min);
 }
 
 // Order phase 1: the bits of F[0, n).
 __device__ __forceinline__ void order_set(const LoopArgs &g, const uint32_t *F, uint32_t n)
 {
-	const uint32_t stride = gridDim.x * blockDim.x;
-	for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-	{
+	block_shares(n, [&](uint64_t i) {
 		const uint32_t t = F[i];
 		if (t < g.T)
 			atomicOr(g.fbits + (t >> 5), 1u << (t & 31));
-	}
+	});
 }
 
 // Order phase 2: the ids back to F, clearing the bits. A warp takes 128 words
@@ -418,8 +495,8 @@ __device__ __forceinline__ void order_write(const LoopArgs &g, uint32_t *__restr
 {
 	const uint32_t lane = lane_id();
 	const uint64_t words = (g.T + 31) / 32;
-	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t stride = ((uint64_t(gridDim.x) * blockDim.x) >> 5) * 128;
+	const uint64_t warp = loop_warp();
+	const uint64_t stride = uint64_t(loop_warps()) * 128;
 	for (uint64_t w0 = warp * 128; w0 < words; w0 += stride)
 	{
 		uint32_t z[4], cnt = 0;
@@ -466,14 +543,13 @@ __device__ __forceinline__ void order_write(const LoopArgs &g, uint32_t *__restr
 template <class Path>
 __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path path)
 {
-	uint32_t phase = 0, target = 0, n = 0, mn = 0;
+	uint32_t phase = 0, n = 0, mn = 0;
 	uint32_t nF = 0, nPrev = 0, cur = 0, level = 0xffffffffu, round = 0, rounds = 0;
-	const uint64_t tid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-	const uint64_t nthreads = uint64_t(gridDim.x) * blockDim.x;
 	const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
 	unsigned long long peeled = 0, ksum = 0, t_start = 0, t_last = 0, ns[4] = {0, 0, 0, 0};
 	if (lead)
 		t_start = t_last = loop_ns();
+	bool ok = true, late = false;
 	auto lap = [&](int kind) {
 		if (lead)
 		{
@@ -481,18 +557,24 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 			ns[kind] += now - t_last;
 			t_last = now;
 			if (now - t_start > LOOP_TIME_LIMIT_NS)
-				atomicExch(&g.ctl->abort, 1u);
+				late = true;
 		}
 	};
-	bool ok = true;
 	while (peeled < g.T)
 	{
+		if (late) // the lead block leaves; the others find it at their next barrier
+			atomicExch(&g.ctl->abort, 1u);
+		if (__syncthreads_or(late))
+		{
+			ok = false;
+			break;
+		}
 		uint32_t *F = cur ? g.F1 : g.F0, *Fp = cur ? g.F0 : g.F1;
 		if (nF == 0)
 		{
 			// level change: level + 1 first, else the minimum of the rest
 			scan_level(g, level + 1, F, &g.ctl->slot[phase & 3]);
-			if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+			if (!(ok = phase_end(g.ctl, phase, n, mn, true)))
 				break;
 			++level;
 			if (lead)
@@ -503,15 +585,14 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 					break; // nothing alive (cannot happen while peeled < T)
 				level = mn;
 				scan_level(g, level, F, &g.ctl->slot[phase & 3]);
-				if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+				if (!(ok = phase_end(g.ctl, phase, n, mn, true)))
 					break;
 			}
 			nF = n;
 			lap(2);
 		}
 		const uint32_t stamp = 0x80000000u | round;
-		for (uint64_t i = tid; i < uint64_t(nF) + nPrev; i += nthreads)
-		{
+		block_shares(uint64_t(nF) + nPrev, [&](uint64_t i) {
 			if (i < nF)
 			{
 				const uint32_t t = F[i];
@@ -523,12 +604,12 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 			}
 			else
 				path.retire(Fp[i - nF]);
-		}
-		if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+		});
+		if (!(ok = phase_end(g.ctl, phase, n, mn, false)))
 			break;
 		lap(0);
 		path.debit(g, F, nF, Fp, &g.ctl->slot[phase & 3], int32_t(level), stamp);
-		if (!(ok = phase_end(g.ctl, phase, target, n, mn)))
+		if (!(ok = phase_end(g.ctl, phase, n, mn, false)))
 			break;
 		lap(1);
 		peeled += nF;
@@ -542,10 +623,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 		{
 			order_set(g, Fp, nF);
 			uint32_t unused, m2;
-			if (!(ok = phase_end(g.ctl, phase, target, unused, m2)))
+			if (!(ok = phase_end(g.ctl, phase, unused, m2, false)))
 				break;
 			order_write(g, Fp, &g.ctl->slot[phase & 3]);
-			if (!(ok = phase_end(g.ctl, phase, target, unused, m2)))
+			if (!(ok = phase_end(g.ctl, phase, unused, m2, false)))
 				break;
 			if (lead)
 				g.ctl->ordered++;
@@ -595,8 +676,9 @@ int run_peel_loop(Ctx &c, LoopBuffers &b, const Path &path, int32_t *S, int32_t 
 	LoopArgs g{b.ctl, S, K, b.R, b.F0, b.F1, b.fbits, c.T, 0xffffffffu};
 	if (tn.sort_shift != NUCLEUS34_TUNE_NEVER)
 		g.sort_min = uint32_t(std::max<uint64_t>(c.T >> tn.sort_shift, 4096));
-	// as many blocks as fit at once, fewer when the scans would leave most of
-	// them without a support word (a barrier costs more the more blocks take part)
+	// as many blocks as fit at once, fewer for small graphs, whose frontiers do
+	// not fill them (a quarter as many blocks: 19% slower on R-MAT scale 12; one
+	// per SM: 17 to 20% slower on the direct variant's graphs of 3M triangles)
 	uint64_t blocks = (c.T + LOOP_THREADS * 4 - 1) / (LOOP_THREADS * 4);
 	blocks = std::min<uint64_t>(std::max<uint64_t>(blocks, 4), uint64_t(per_sm) * uint64_t(c.sm_count));
 	cudaLaunchConfig_t cfg{};
