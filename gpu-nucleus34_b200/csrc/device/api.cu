@@ -316,6 +316,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	Incidence inc;
 	CliqueCsr csr;
 	BitMats mats;
+	InMats in;
 	int32_t *S = nullptr;
 	uint32_t *own = nullptr;
 	int rc = NUCLEUS34_OK;
@@ -344,15 +345,13 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 		c.lean_run = false;
 		// the on-demand variant runs on the listing's bit matrices when they
 		// were kept and the rest fits beside them, else on the incidence lists
-		const bool bits = c.T && bit_form_fits(c, mats);
+		bool bits = c.T && mats.cells;
+		if (bits && (rc = build_in_rows(c, mats, in, &bits)))
+			break;
 		if (!bits)
 			free_mats(c, mats);
 		if (bits)
-		{
-			if ((rc = build_in_lists(c, mats, inc)))
-				break;
-			r.sum_te_sq = inc.sum_te_sq;
-		}
+			r.sum_te_sq = in.sum_te_sq;
 		else if (c.T)
 		{
 			// The on-demand peel with death flags (T < 2^30) uses either the
@@ -381,7 +380,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (variant == NUCLEUS34_DIRECT && (rc = dalloc(c, &own, c.T, "clique owner counts")))
 				break;
-			if ((rc = bits ? count_support_bits(c, mats, inc, S, &total) : count_support(c, inc, S, &total, own)))
+			if ((rc = bits ? count_support_bits(c, mats, in, S, &total) : count_support(c, inc, S, &total, own)))
 				break;
 			if (total % 4)
 			{
@@ -431,7 +430,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 			if (total)
 			{
 				rc = variant == NUCLEUS34_DIRECT ? peel_direct(c, csr, S, c.dK, &pc)
-					 : bits						 ? peel_bits(c, mats, inc, S, c.dK, &pc)
+					 : bits						 ? peel_bits(c, mats, in, S, c.dK, &pc)
 												 : peel(c, inc, S, c.dK, &pc);
 				if (rc)
 					break;
@@ -450,6 +449,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	free_incidence(c, inc);
 	free_clique_csr(c, csr);
 	free_mats(c, mats);
+	free_in_rows(c, in);
 	c.release(S);
 	c.release(own);
 	if (rc)

@@ -11,18 +11,18 @@
 //     that have source u are the set bits of row v AND row w: 32 candidates
 //     per word pair, no list and no search. The peel clears the bits of dead
 //     triangles, so a candidate's two triangles of source u are known to live.
-//   - by its fourth ("top") triangle (v, w, x), whose cliques {u; v, w, x} are
-//     the common sources of two of the in-lists of its three edges (the
-//     in-list of v -> w: the sources u of the triangles (u, v, w), ascending,
-//     with their ids). T entries in all, a third of the incidence.
-// Every clique is in three row ANDs and one list intersection. The ids of the
+//   - by its fourth ("top") triangle (v, w, x). In its names (u -> v -> w, with
+//     x = y the clique's source): the in-row of edge u -> v has a bit for every
+//     in-edge y -> u with a triangle (y, u, v), the in-row of u -> w one for
+//     every (y, u, w), so the cliques are again the set bits of two rows.
+// Every clique is in three row ANDs and one AND of in-rows. The ids of the
 // partners come from the cells (a word's first id + the bits below), and the
 // last one, which is not in hand, from the cell of its own source: the c edges
-// of the two triangles found tell its row and its position. So a clique costs
-// a fixed chain of loads, where the lists needed a binary search of the longest
-// list, and of the in-lists the peel reads little: a live-entry bitmap and a
-// live count per edge pass over the dead (R-MAT scale 18: 5.8e7 entries looked
-// up in all, of 4.8e9 in the lists of the dying).
+// of the two triangles found (their a edges, for the in-rows) tell its row and
+// its position. So a clique costs a fixed chain of loads, where the lists
+// needed a binary search of the longest list. An in-row whose triangles are all
+// dead is passed by a count (R-MAT scale 18: 5.8e7 bits taken up, where the
+// in-lists of the dying hold 4.8e9 entries).
 //
 // What bounds the debit: scattered accesses. Of a clique's three atomics and
 // about five gathers, the third partner's cell and support are nowhere near
@@ -44,186 +44,223 @@ namespace {
 
 constexpr int SUP_THREADS = 256;
 
-// The two shorter of a triangle's three in-lists: A, to be looked up in B.
-// Roles: 0 = under b (u -> v), 1 = under a (u -> w), 2 = under c (v -> w).
-struct InPair
-{
-	uint32_t a0, a1, b0, b1;
-	uint32_t ra, rb;
-};
+// ---- in-rows -----------------------------------------------------------------
 
-__device__ __forceinline__ InPair in_pair(uint2 sb, uint2 sa, uint2 sc)
+// column of every edge among its head's in-edges, and the in-degrees
+__global__ void k_in_columns(const uint32_t *__restrict__ E, uint64_t m, uint32_t *__restrict__ indeg,
+							 uint4 *__restrict__ erec)
 {
-	uint2 p = sb, q = sa, r = sc;
-	uint32_t rp = 0, rq = 1, rr = 2;
-	uint2 t;
-	uint32_t rt;
-	if (q.y - q.x < p.y - p.x)
-	{
-		t = p; p = q; q = t;
-		rt = rp; rp = rq; rq = rt;
-	}
-	if (r.y - r.x < q.y - q.x)
-	{
-		t = q; q = r; r = t;
-		rt = rq; rq = rr; rr = rt;
-	}
-	if (q.y - q.x < p.y - p.x)
-	{
-		t = p; p = q; q = t;
-		rt = rp; rp = rq; rq = rt;
-	}
-	return InPair{p.x, p.y, q.x, q.y, rp, rq};
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
+		erec[e].w = atomicAdd(indeg + E[e], 1u);
 }
 
-// support[t] = cliques on t. A warp takes 32 triangles: each lane counts the
-// row ANDs of its own triangle (neighbours share their source, so the rows
-// come from L1); the in-list entries of all 32 are then dealt out to the
-// lanes one by one, each a binary search in the other list.
-__global__ void __launch_bounds__(SUP_THREADS) k_support_bits(
-	const uint32_t *__restrict__ tris, uint64_t T, const uint2 *__restrict__ erec, const uint4 *__restrict__ cells,
-	const uint2 *__restrict__ span, const uint32_t *__restrict__ third, int32_t *__restrict__ support,
-	unsigned long long *__restrict__ total)
+// cells of every edge's in-row
+__global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
+							uint32_t *__restrict__ width)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
+		width[e] = (indeg[src[e]] + 31) >> 5;
+}
+
+__global__ void k_in_starts(const uint64_t *__restrict__ off, uint64_t m, uint4 *__restrict__ erec)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
+		erec[e].z = uint32_t(off[e]);
+}
+
+// the bit of every triangle (y, u, v): in-row of c = u -> v, column of b = y -> u
+__global__ void k_in_set(const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec,
+						 uint4 *__restrict__ cells)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
+	{
+		const uint32_t col = __ldg(&erec[tris[3 * t + 1]].w), row = __ldg(&erec[tris[3 * t + 2]].z);
+		atomicOr(&cells[row + (col >> 5)].x, 1u << (col & 31));
+	}
+}
+
+// triangles per in-row, and the sum over edges of (triangles on the edge)^2:
+// those with the edge as a or b are in its symmetric row
+__global__ void k_in_counts(const uint4 *__restrict__ erec, uint64_t m, const uint4 *__restrict__ rows,
+							const uint4 *__restrict__ cells, const uint32_t *__restrict__ width,
+							uint32_t *__restrict__ cnt, uint2 *__restrict__ live,
+							unsigned long long *__restrict__ sum_sq)
+{
+	unsigned long long acc = 0;
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
+	{
+		const uint4 r = erec[e];
+		const uint32_t W = width[e];
+		uint32_t n = 0;
+		for (uint32_t q = 0; q < W; ++q)
+			n += __popc(cells[r.z + q].x);
+		cnt[e] = n;
+		live[e] = make_uint2(n, W);
+		unsigned long long d = n;
+		for (uint32_t q = 0; q < (r.y >> 16); ++q)
+			d += __popc(rows[r.x + q].z);
+		acc += d * d;
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		acc += __shfl_xor_sync(FULL, acc, o);
+	if (lane_id() == 0 && acc)
+		atomicAdd(sum_sq, acc);
+}
+
+// first positions of the cells' triangles in tri; all not dead, none dying. A
+// warp takes 32 edges, whose in-rows lie behind one another, as their triangles
+// do in tri: a running sum over their cells (one thread per edge wrote them at
+// scattered places: 3.2 ms on R-MAT scale 18, 0.3 now).
+__global__ void k_in_firsts(const uint4 *__restrict__ erec, uint64_t m, const uint32_t *__restrict__ width,
+							const uint64_t *__restrict__ off, uint4 *__restrict__ cells)
 {
 	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 	const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
 	const uint32_t lane = lane_id();
-	unsigned long long acc = 0;
-	for (uint64_t base = warp * 32; base < T; base += nwarps * 32)
+	for (uint64_t e0 = warp * 32; e0 < m; e0 += nwarps * 32)
 	{
-		const uint64_t t = base + lane;
-		uint32_t cnt = 0;
-		InPair L{0, 0, 0, 0, 0, 0};
-		if (t < T)
+		const uint64_t last = min(e0 + 32, m) - 1;
+		const uint32_t first = erec[e0].z, end = erec[last].z + width[last];
+		uint32_t at = uint32_t(off[e0]);
+		for (uint32_t w0 = first; w0 < end; w0 += 32)
 		{
-			const uint32_t a = __ldg(tris + 3 * t), b = __ldg(tris + 3 * t + 1), c = __ldg(tris + 3 * t + 2);
-			const uint2 ra = __ldg(erec + a), rb = __ldg(erec + b);
-			const uint32_t W = ra.y >> 16;
-			for (uint32_t q = 0; q < W; ++q)
-				cnt += __popc(__ldg(&cells[ra.x + q].z) & __ldg(&cells[rb.x + q].z));
-			L = in_pair(__ldg(span + b), __ldg(span + a), __ldg(span + c));
-		}
-		const uint32_t len = L.a1 - L.a0;
-		const uint32_t incl = warp_incl_scan(len), excl = incl - len;
-		const uint32_t items = __shfl_sync(FULL, incl, 31);
-		for (uint32_t k0 = 0; k0 < items; k0 += 32)
-		{
-			const uint32_t k = k0 + lane;
-			const uint32_t s = warp_owner(incl, k);
-			const uint32_t i = __shfl_sync(FULL, L.a0, s) + k - __shfl_sync(FULL, excl, s);
-			const uint32_t b0 = __shfl_sync(FULL, L.b0, s), b1 = __shfl_sync(FULL, L.b1, s);
-			bool found = false;
-			if (k < items)
+			const uint32_t w = w0 + lane, x = w < end ? cells[w].x : 0u, n = __popc(x);
+			uint32_t sum = n; // inclusive over the lanes
+#pragma unroll
+			for (uint32_t o = 1; o < 32; o <<= 1)
 			{
-				const uint32_t x = __ldg(third + i);
-				const uint32_t p = lower_bound32(third, b0, b1, x);
-				found = p < b1 && __ldg(third + p) == x;
+				const uint32_t y = __shfl_up_sync(FULL, sum, o);
+				if (lane >= o)
+					sum += y;
 			}
-			// each lane takes the matches among its own triangle's items
-			const uint32_t fm = __ballot_sync(FULL, found);
-			const uint32_t lo = excl > k0 ? excl - k0 : 0u, hi = incl > k0 ? incl - k0 : 0u;
-			if (lo < 32 && hi > lo)
-				cnt += __popc(fm & ((hi >= 32 ? FULL : (1u << hi) - 1u) & ~((1u << lo) - 1u)));
+			if (w < end)
+				cells[w] = make_uint4(x, at + sum - n, x, 0u);
+			at += __shfl_sync(FULL, sum, 31);
 		}
-		if (t < T)
-			support[t] = int32_t(cnt);
+	}
+}
+
+__global__ void k_in_place(const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec,
+						   const uint4 *__restrict__ cells, uint32_t *__restrict__ tri)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
+	{
+		const uint32_t col = __ldg(&erec[tris[3 * t + 1]].w), row = __ldg(&erec[tris[3 * t + 2]].z);
+		const uint2 c = __ldg(reinterpret_cast<const uint2 *>(cells + row + (col >> 5)));
+		tri[c.y + __popc(c.x & ((1u << (col & 31)) - 1u))] = uint32_t(t);
+	}
+}
+
+// ---- support -------------------------------------------------------------------
+
+// support[t] = cliques on t: the common bits of its two rows and of its two
+// in-rows, one thread per triangle (neighbours share their source, so the rows
+// come from L1).
+__global__ void __launch_bounds__(SUP_THREADS) k_support_bits(
+	const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
+	const uint4 *__restrict__ in_rows, const uint2 *__restrict__ in_live, int32_t *__restrict__ support,
+	unsigned long long *__restrict__ total)
+{
+	unsigned long long acc = 0;
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
+	{
+		const uint32_t a = __ldg(tris + 3 * t), b = __ldg(tris + 3 * t + 1);
+		const uint4 ra = __ldg(erec + a), rb = __ldg(erec + b);
+		const uint2 la = __ldg(in_live + a), lb = __ldg(in_live + b);
+		uint32_t cnt = 0;
+		for (uint32_t q = 0; q < (ra.y >> 16); ++q)
+			cnt += __popc(__ldg(&rows[ra.x + q].z) & __ldg(&rows[rb.x + q].z));
+		if (la.x && lb.x)
+			for (uint32_t q = 0; q < la.y; ++q)
+				cnt += __popc(__ldg(&in_rows[ra.z + q].x) & __ldg(&in_rows[rb.z + q].x));
+		support[t] = int32_t(cnt);
 		acc += cnt;
 	}
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1)
 		acc += __shfl_xor_sync(FULL, acc, o);
-	if (lane == 0 && acc)
+	if (lane_id() == 0 && acc)
 		atomicAdd(total, acc);
 }
 
-// crec[t] = record of t's c edge
-__global__ void k_c_records(const uint32_t *__restrict__ tris, uint64_t T, const uint2 *__restrict__ erec,
+// ---- peel ----------------------------------------------------------------------
+
+// crec[t] = record of t's c edge: its row and position
+__global__ void k_c_records(const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec,
 							uint2 *__restrict__ crec)
 {
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
-		crec[t] = __ldg(erec + __ldg(tris + 3 * t + 2));
-}
-
-// live[e] = entries of e's in-list
-__global__ void k_in_lengths(const uint2 *__restrict__ span, uint64_t m, uint32_t *__restrict__ live)
-{
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
-		live[e] = span[e].y - span[e].x;
-}
-
-// tpos[t] = position of t's in-list entry
-__global__ void k_in_positions(const uint32_t *__restrict__ tri, uint64_t T, uint32_t *__restrict__ tpos)
-{
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < T; i += stride)
-		tpos[tri[i]] = uint32_t(i);
+		crec[t] = __ldg(reinterpret_cast<const uint2 *>(erec + __ldg(tris + 3 * t + 2)));
 }
 
 struct BitPath
 {
-	const uint32_t *tris, *src;
-	const uint2 *erec;
+	const uint32_t *tris;
+	const uint4 *erec;
 	uint4 *cells;
-	const uint2 *span;
-	const uint32_t *third, *tri;
-	uint32_t *inlive;     // per edge: in-list entries whose triangle is not dead
-	uint32_t *inbits;     // bit per in-list entry: its triangle is not dead
-	const uint32_t *tpos; // position of each triangle's in-list entry, or null (then searched)
-	const uint2 *crec;    // record of each triangle's c edge, or null (then looked up through tris)
+	uint4 *in_cells;
+	const uint32_t *in_tri;
+	uint2 *in_live;
+	const uint2 *crec; // record of each triangle's c edge, or null (then looked up through tris)
 
+	// Sets (mark) or clears (retire) the two bits of t in its source's matrix
+	// and its bit in the in-row of its c edge.
 	__device__ __forceinline__ void mark(uint32_t t) const
 	{
-		const uint2 ra = __ldg(erec + __ldg(tris + 3 * uint64_t(t))),
-					rb = __ldg(erec + __ldg(tris + 3 * uint64_t(t) + 1));
-		const uint32_t p = ra.y & 0xffffu, j = rb.y & 0xffffu;
+		const uint32_t b = __ldg(tris + 3 * uint64_t(t) + 1), c = __ldg(tris + 3 * uint64_t(t) + 2);
+		const uint4 ra = __ldg(erec + __ldg(tris + 3 * uint64_t(t))), rb = __ldg(erec + b);
+		const uint32_t in = __ldg(&erec[c].z), p = ra.y & 0xffffu, j = rb.y & 0xffffu, col = rb.w;
 		atomicOr(&cells[ra.x + (j >> 5)].w, 1u << (j & 31));
 		atomicOr(&cells[rb.x + (p >> 5)].w, 1u << (p & 31));
+		atomicOr(&in_cells[in + (col >> 5)].w, 1u << (col & 31));
 	}
 
 	__device__ __forceinline__ void retire(uint32_t t) const
 	{
-		const uint32_t b = __ldg(tris + 3 * uint64_t(t) + 1);
-		const uint2 ra = __ldg(erec + __ldg(tris + 3 * uint64_t(t))), rb = __ldg(erec + b);
-		const uint32_t p = ra.y & 0xffffu, j = rb.y & 0xffffu;
+		const uint32_t b = __ldg(tris + 3 * uint64_t(t) + 1), c = __ldg(tris + 3 * uint64_t(t) + 2);
+		const uint4 ra = __ldg(erec + __ldg(tris + 3 * uint64_t(t))), rb = __ldg(erec + b);
+		const uint32_t in = __ldg(&erec[c].z), p = ra.y & 0xffffu, j = rb.y & 0xffffu, col = rb.w;
 		atomicAnd(&cells[ra.x + (j >> 5)].z, ~(1u << (j & 31)));
 		atomicAnd(&cells[rb.x + (p >> 5)].z, ~(1u << (p & 31)));
-		const uint32_t c = __ldg(tris + 3 * uint64_t(t) + 2);
-		atomicSub(inlive + c, 1u);
-		uint32_t i;
-		if (tpos)
-			i = __ldg(tpos + t);
-		else
-		{
-			const uint2 sc = __ldg(span + c);
-			i = lower_bound32(third, sc.x, sc.y, __ldg(src + b));
-		}
-		atomicAnd(inbits + (i >> 5), ~(1u << (i & 31)));
+		atomicAnd(&in_cells[in + (col >> 5)].z, ~(1u << (col & 31)));
+		atomicSub(&in_live[c].x, 1u);
+	}
+
+	__device__ __forceinline__ uint2 row_of(uint32_t e) const
+	{
+		return __ldg(reinterpret_cast<const uint2 *>(erec + e));
 	}
 
 	__device__ __forceinline__ uint2 c_record(uint32_t t) const
 	{
-		return __ldg(erec + __ldg(tris + 3 * uint64_t(t) + 2));
+		return crec ? __ldg(crec + t) : row_of(__ldg(tris + 3 * uint64_t(t) + 2));
 	}
 
 	// Cliques found, up to 32 at a time, one per lane when they are settled:
 	// HEAD_V / HEAD_W: x -> v / x -> w; DIES_1 / DIES_2: the partner (u, v, x) /
-	// (u, w, x) dies this round; LIST: found in the in-lists.
-	static constexpr uint32_t HEAD_V = 4, HEAD_W = 8, DIES_1 = 16, DIES_2 = 32, LIST = 64;
+	// (u, w, x) dies this round; IN: found in the in-rows.
+	static constexpr uint32_t HEAD_V = 4, HEAD_W = 8, DIES_1 = 16, DIES_2 = 32, IN = 64;
 	struct Batch
 	{
-		// slot << 8 | flags, position of x / role pair, two partners (as far as known)
+		// slot << 8 | flags, position of x, two partners (as far as known; IN:
+		// their positions in in_tri)
 		uint32_t flags[32], ix[32], id1[32], id2[32];
 	};
 	struct WarpMem
 	{
 		Batch batch;
-		// the triangles of the batch in hand: {id, first cells of the rows of
-		// its head w and tail v, first word of list A as an entry}, {W << 16 |
-		// position of w, role pair and order << 16 | position of v, list B}
-		uint4 s0[32], s1[32];
-		uint32_t q0[32], q1[32]; // list entries dealt out: triangle, entry
+		// the triangles of the unit in hand: {id, first cell of the row of its
+		// head w, W << 16 | position of w, position of v}
+		uint4 slot[32];
 		uint32_t next[Appender::CAP];
 	};
 	static constexpr uint32_t SMEM = uint32_t(sizeof(WarpMem)) * LOOP_WARPS;
@@ -242,41 +279,22 @@ struct BitPath
 		int32_t *S;
 		Appender next;
 		int32_t level;
-		uint32_t stamp;
 		uint32_t queued; // cliques in the batch
 
 		__device__ __forceinline__ Settler(const BitPath &path, WarpMem &mem, const LoopArgs &g, uint32_t *Fn,
-										   PhaseSlot *slot, int32_t lv, uint32_t st)
-			: p(path), m(mem), S(g.S), next{mem.next, Fn, &slot->n, &g.ctl->c.error, g.T, 0u}, level(lv), stamp(st),
-			  queued(0)
+										   PhaseSlot *slot, int32_t lv)
+			: p(path), m(mem), S(g.S), next{mem.next, Fn, &slot->n, &g.ctl->c.error, g.T, 0u}, level(lv), queued(0)
 		{
 		}
 
-		// A clique found in the rows, at place `at` of the batch: slot s, x at
-		// position ix; id1 and id2 as far as v's and w's row tell them.
-		__device__ __forceinline__ void put_row(uint32_t at, uint32_t s, uint32_t ix, uint32_t flags, uint32_t id1,
-												uint32_t id2)
+		// A clique found, at place `at` of the batch.
+		__device__ __forceinline__ void put(uint32_t at, uint32_t slot, uint32_t ix, uint32_t flags, uint32_t id1,
+											uint32_t id2)
 		{
-			m.batch.flags[at] = s << 8 | flags;
+			m.batch.flags[at] = slot << 8 | flags;
 			m.batch.ix[at] = ix;
 			m.batch.id1[at] = id1;
 			m.batch.id2[at] = id2;
-		}
-
-		// A match of two in-lists: partners id1 and id2 of slot s's triangle, by
-		// role pair. With two of the triangles (y, u, v), (y, u, w), (y, v, w) of y
-		// in hand, the edges of y in them give the row and the position of the
-		// third: uv + uw (0): head y -> w, tail y -> v, their a edges; uv + vw (1):
-		// head y -> w from vw's a, tail y -> u from uv's b; uw + vw (2): head
-		// y -> v from vw's b, tail y -> u from uw's b.
-		__device__ __forceinline__ void put_list(uint32_t at, uint32_t s, uint32_t kind, uint32_t id1, uint32_t id2)
-		{
-			put_row(at, s, kind, LIST, id1, id2);
-		}
-
-		__device__ __forceinline__ uint2 c_rec(uint32_t t) const
-		{
-			return p.crec ? __ldg(p.crec + t) : p.c_record(t);
 		}
 
 		// Settles the batch: one clique per lane. All lanes call.
@@ -291,22 +309,27 @@ struct BitPath
 				const uint32_t f = m.batch.flags[lane], ix = m.batch.ix[lane];
 				id1 = m.batch.id1[lane];
 				id2 = m.batch.id2[lane];
-				const uint4 a = m.s0[f >> 8];
+				const uint4 a = m.slot[f >> 8];
 				t = a.x;
-				uint2 h, l;
-				if (f & LIST)
+				live1 = !(f & DIES_1);
+				live2 = !(f & DIES_2);
+				uint2 h = make_uint2(0, 0), l = h;
+				if (f & IN)
 				{
-					const int32_t s1 = ld_support(S + id1), s2 = ld_support(S + id2);
-					l = __ldg(p.erec + __ldg(p.tris + 3 * uint64_t(id1) + (ix == 0 ? 0 : 1)));
-					h = __ldg(p.erec + __ldg(p.tris + 3 * uint64_t(id2) + (ix == 2 ? 1 : 0)));
-					live1 = s1 >= 0;
-					live2 = s2 >= 0;
-					ok = !partner_blocks(s1, id1, t, stamp) && !partner_blocks(s2, id2, t, stamp);
+					// (y, u, v) and (y, u, w): their a edges are tail y -> v and head
+					// y -> w of the third, (y, v, w)
+					id1 = __ldg(p.in_tri + id1);
+					id2 = __ldg(p.in_tri + id2);
+					ok = (live1 || id1 > t) && (live2 || id2 > t);
+					if (ok)
+					{
+						l = p.row_of(__ldg(p.tris + 3 * uint64_t(id1)));
+						h = p.row_of(__ldg(p.tris + 3 * uint64_t(id2)));
+					}
 				}
 				else
 				{
-					const uint4 b = m.s1[f >> 8];
-					const uint32_t W = b.x >> 16, pw = b.x & 0xffffu, pv = b.y & 0xffffu;
+					const uint32_t W = a.z >> 16, pw = a.z & 0xffffu, pv = a.w;
 					// (plain loads: the state words beside the ids change between phases)
 					const uint4 *row_x = p.cells + (a.y + (ix - pw) * W);
 					const bool xv = f & HEAD_V, xw = f & HEAD_W;
@@ -319,15 +342,12 @@ struct BitPath
 						id1 = rv.y + __popc(rv.x & ((1u << (pv & 31)) - 1u));
 					if (!xw)
 						id2 = rw.y + __popc(rw.x & ((1u << (pw & 31)) - 1u));
-					live1 = !(f & DIES_1);
-					live2 = !(f & DIES_2);
 					ok = (xv || (rv.x >> (pv & 31)) & 1u) && (xw || (rw.x >> (pw & 31)) & 1u);
-					h = l = make_uint2(0, 0);
 					if (ok)
 					{
 						// x -> v: head x -> w, tail x -> v; v -> x -> w: head v -> w
 						// (t's own c edge), tail v -> x; v -> w -> x: the reverse
-						const uint2 r1 = c_rec(id1), r2 = c_rec(xv ? id2 : t);
+						const uint2 r1 = p.c_record(id1), r2 = p.c_record(xv ? id2 : t);
 						h = xv || xw ? r2 : r1;
 						l = xv || xw ? r1 : r2;
 					}
@@ -398,55 +418,56 @@ struct BitPath
 		}
 	}
 
-	// A warp takes a batch of consecutive frontier triangles, one per lane for
-	// the loads of their records. The words of their row pairs, and then the
-	// live entries of their shortest in-lists, are dealt out to the lanes across
-	// the batch; the cliques found go through the found.
+	// A warp takes a unit of consecutive frontier triangles, one per lane for
+	// the loads of their records. The words of their row pairs, and then of
+	// their pairs of in-rows, are dealt out to the lanes across the unit; the
+	// cliques found are settled 32 at a time, one lane per clique.
 	__device__ __forceinline__ void debit(const LoopArgs &g, const uint32_t *F, uint32_t nF, uint32_t *Fn, PhaseSlot *slot,
-										  int32_t level, uint32_t stamp) const
+										  int32_t level) const
 	{
 		extern __shared__ uint4 loop_smem[];
 		WarpMem &m = reinterpret_cast<WarpMem *>(loop_smem)[threadIdx.x >> 5];
-		Settler found(*this, m, g, Fn, slot, level, stamp);
+		Settler found(*this, m, g, Fn, slot, level);
 		const uint32_t lane = lane_id();
-		const Units u = debit_units(nF, (gridDim.x * blockDim.x) >> 5);
+		const Units u = debit_units(nF, loop_warps());
 		claim_units(u.total, &slot->work, [&](uint32_t unit) {
 			const uint32_t stripe = unit & ((1u << u.shift) - 1u);
 			const uint32_t base = (unit >> u.shift) * u.ch;
-			const bool have = lane < u.ch && base + lane < nF;
-			uint32_t row_w = 0, row_v = 0, W = 0, pos = 0;
-			uint2 la = make_uint2(0, 0); // in-list A
-			if (have)
+			uint32_t row_w = 0, row_v = 0, W = 0, pos = 0, in_w = 0, in_v = 0, Win = 0;
+			if (lane < u.ch && base + lane < nF)
 			{
 				const uint32_t t = F[base + lane];
 				const uint32_t a = __ldg(tris + 3 * uint64_t(t)), b = __ldg(tris + 3 * uint64_t(t) + 1),
 							   c = __ldg(tris + 3 * uint64_t(t) + 2);
-				const uint2 ra = __ldg(erec + a), rb = __ldg(erec + b);
-				// the two in-lists with the fewest live entries, the least first
-				// (role 0: under b, 1: under a, 2: under c); none live, no clique
-				const uint32_t nb = inlive[b], na = inlive[a], nc = inlive[c];
+				const uint4 ra = __ldg(erec + a), rb = __ldg(erec + b);
+				// none live under one of the edges: no clique through the in-rows
+				const uint2 lb = in_live[b];
+				const uint32_t na = in_live[a].x, nc = in_live[c].x;
 				row_w = ra.x;
 				row_v = rb.x;
 				W = ra.y >> 16;
 				pos = ra.y << 16 | (rb.y & 0xffffu);
-				uint32_t meta = 0;
-				uint2 lb = la;
-				if (min(min(na, nb), nc))
-				{
-					const uint32_t most = nc >= na && nc >= nb ? 2u : (na >= nb ? 1u : 0u);
-					// the pair without `most`: lower role first, swapped if the other has fewer
-					const uint32_t e0 = most == 0 ? a : b, e1 = most == 2 ? a : c;
-					const bool swap = (most == 0 ? na : nb) > (most == 2 ? na : nc);
-					la = __ldg(span + (swap ? e1 : e0));
-					lb = __ldg(span + (swap ? e0 : e1));
-					// role pair 0: uv + uw, 1: uv + vw, 2: uw + vw; swap: A holds the higher role
-					meta = (2 - most) << 1 | (swap ? 1u : 0u);
-				}
-				m.s0[lane] = make_uint4(t, ra.x, rb.x, la.x & ~31u);
-				m.s1[lane] = make_uint4(ra.y, (rb.y & 0xffffu) | meta << 16, lb.x, lb.y);
+				in_w = ra.z;
+				in_v = rb.z;
+				Win = min(min(lb.x, na), nc) ? lb.y : 0u;
+				m.slot[lane] = make_uint4(t, ra.x, ra.y, rb.y & 0xffffu);
 			}
 			__syncwarp();
 			uint4 cw = make_uint4(0, 0, 0, 0), cv = cw; // this lane's word pair
+			auto put = [&](uint32_t o, uint32_t s, uint32_t ix, uint32_t bit, bool mine, uint32_t kind) {
+				const uint32_t vx = __shfl_sync(FULL, cv.x, o), vy = __shfl_sync(FULL, cv.y, o),
+							   vd = __shfl_sync(FULL, cv.w, o);
+				const uint32_t wx = __shfl_sync(FULL, cw.x, o), wy = __shfl_sync(FULL, cw.y, o),
+							   wd = __shfl_sync(FULL, cw.w, o);
+				if (!mine)
+					return;
+				const uint32_t below = (1u << bit) - 1u;
+				found.put(lane, s, ix,
+						  kind | ((vx >> bit) & 1u ? HEAD_V : 0u) | ((wx >> bit) & 1u ? HEAD_W : 0u) |
+							  ((vd >> bit) & 1u ? DIES_1 : 0u) | ((wd >> bit) & 1u ? DIES_2 : 0u),
+						  vy + __popc(vx & below), wy + __popc(wx & below));
+			};
+			auto full = [&]() { found.settle(); };
 			deal_bits(
 				W, u.ch == 1, stripe, u.shift, found.queued,
 				[&](uint32_t s, uint32_t q, bool on) {
@@ -464,89 +485,24 @@ struct BitPath
 					const uint32_t low_w = (cw.x & below_j) | (~cw.x & below_p);
 					return cw.z & cv.z & ~(cv.w & low_v) & ~(cw.w & low_w);
 				},
-				[&](uint32_t o, uint32_t s, uint32_t ix, uint32_t bit, bool mine) {
-					const uint32_t vx = __shfl_sync(FULL, cv.x, o), vy = __shfl_sync(FULL, cv.y, o),
-								   vd = __shfl_sync(FULL, cv.w, o);
-					const uint32_t wx = __shfl_sync(FULL, cw.x, o), wy = __shfl_sync(FULL, cw.y, o),
-								   wd = __shfl_sync(FULL, cw.w, o);
-					if (!mine)
-						return;
-					const uint32_t below = (1u << bit) - 1u;
-					found.put_row(lane, s, ix,
-								 ((vx >> bit) & 1u ? HEAD_V : 0u) | ((wx >> bit) & 1u ? HEAD_W : 0u) |
-									 ((vd >> bit) & 1u ? DIES_1 : 0u) | ((wd >> bit) & 1u ? DIES_2 : 0u),
-								 vy + __popc(vx & below), wy + __popc(wx & below));
-				},
-				[&]() { found.settle(); });
-			// entries [a0, a1) as bits of the words that hold them
-			const uint32_t nw = la.y > la.x ? ((la.y - 1) >> 5) - (la.x >> 5) + 1 : 0u;
-			if (!__any_sync(FULL, nw != 0))
-			{
-				if (found.queued)
-					found.settle();
-				__syncwarp(); // the slots are rewritten by the next batch
-				return;
-			}
-			uint32_t dealt = 0;
-			auto search = [&]() {
-				__syncwarp();
-				bool live = false;
-				uint32_t ia = 0, ib = 0, s = 0;
-				if (lane < dealt)
-				{
-					s = m.q0[lane];
-					const uint32_t i = m.s0[s].w + m.q1[lane], x = __ldg(third + i);
-					const uint32_t b1 = m.s1[s].w, p = lower_bound32(third, m.s1[s].z, b1, x);
-					if (p < b1 && __ldg(third + p) == x)
-					{
-						live = (inbits[p >> 5] >> (p & 31)) & 1u;
-						ia = __ldg(tri + i);
-						ib = __ldg(tri + p);
-					}
-				}
-				dealt = 0;
-				const uint32_t lm = __ballot_sync(FULL, live);
-				const uint32_t at = found.queued + __popc(lm & lanemask_lt()), sum = found.queued + __popc(lm);
-				const uint32_t meta = m.s1[s].y >> 16;
-				if (live && at < 32)
-					found.put_list(at, s, meta >> 1, meta & 1u ? ib : ia, meta & 1u ? ia : ib);
-				found.queued = min(sum, 32u);
-				if (sum >= 32)
-				{
-					found.settle();
-					if (live && at >= 32)
-						found.put_list(at - 32, s, meta >> 1, meta & 1u ? ib : ia, meta & 1u ? ia : ib);
-					found.queued = sum - 32;
-				}
-				__syncwarp();
-			};
-			deal_bits(
-				nw, u.ch == 1, stripe, u.shift, dealt,
-				[&](uint32_t s, uint32_t q, bool on) {
-					const uint32_t a0 = __shfl_sync(FULL, la.x, s), a1 = __shfl_sync(FULL, la.y, s);
-					if (!on)
-						return 0u;
-					const uint32_t w = (a0 >> 5) + q;
-					uint32_t z = inbits[w];
-					if (q == 0)
-						z &= FULL << (a0 & 31);
-					if (a1 - w * 32 < 32)
-						z &= (1u << (a1 & 31)) - 1u;
-					return z;
-				},
-				[&](uint32_t, uint32_t s, uint32_t i, uint32_t, bool mine) {
-					if (mine)
-					{
-						m.q0[lane] = s;
-						m.q1[lane] = i;
-					}
-				},
-				search);
-			if (dealt)
-				search();
+				[&](uint32_t o, uint32_t s, uint32_t ix, uint32_t bit, bool mine) { put(o, s, ix, bit, mine, 0u); },
+				full);
+			if (__any_sync(FULL, Win != 0))
+				deal_bits(
+					Win, u.ch == 1, stripe, u.shift, found.queued,
+					[&](uint32_t s, uint32_t q, bool on) {
+						const uint32_t rw = __shfl_sync(FULL, in_w, s), rv = __shfl_sync(FULL, in_v, s);
+						if (!on)
+							return 0u;
+						cw = in_cells[rw + q];
+						cv = in_cells[rv + q];
+						return cw.z & cv.z;
+					},
+					[&](uint32_t o, uint32_t s, uint32_t ix, uint32_t bit, bool mine) { put(o, s, ix, bit, mine, IN); },
+					full);
 			if (found.queued)
 				found.settle();
-			__syncwarp(); // the slots are rewritten by the next batch
+			__syncwarp(); // the slots are rewritten by the next unit
 		});
 		found.next.finish();
 	}
@@ -565,15 +521,94 @@ bool bit_form_wanted(const Ctx &c, int variant)
 	return variant == NUCLEUS34_ONDEMAND && !(c.opt_flags & LIST_FORM);
 }
 
-// Room for the in-lists (8 bytes per triangle), support, k and two frontiers
-// (16), the two bitmaps, and the per-edge arrays of the in-list build.
-bool bit_form_fits(const Ctx &c, const BitMats &mats)
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits)
 {
-	const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
-	return mats.cells && 24 * c.T + c.T / 4 + 28 * c.m + (uint64_t(1) << 20) <= room;
+	const uint64_t T = c.T, m = c.m;
+	*fits = false;
+	uint32_t *indeg = nullptr, *width = nullptr, *cnt = nullptr;
+	uint64_t *off = nullptr;
+	unsigned long long *sumsq = nullptr;
+	const uint32_t gm = grid_for(c, m, 256), gt = grid_for(c, T, 256);
+	int rc = NUCLEUS34_OK;
+	do
+	{
+		if ((rc = dalloc(c, &indeg, c.n, "in-degrees")) || (rc = dalloc(c, &width, m, "in-row widths")) ||
+			(rc = dalloc(c, &off, m + 1, "in-row offsets")))
+			break;
+		if (cudaMemsetAsync(indeg, 0, c.n * 4, c.stream) != cudaSuccess)
+		{
+			rc = fail(NUCLEUS34_E_CUDA, "memset");
+			break;
+		}
+		k_in_columns<<<gm, 256, 0, c.stream>>>(c.dE, m, indeg, mats.erec);
+		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dsrc, m, indeg, width);
+		c.launches += 2;
+		c.release(indeg);
+		indeg = nullptr;
+		if ((rc = scan_u32(c, width, off, m)))
+			break;
+		if (cudaMemcpyAsync(&in.nwords, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaStreamSynchronize(c.stream) != cudaSuccess)
+		{
+			rc = fail(NUCLEUS34_E_CUDA, "in-row widths");
+			break;
+		}
+		// the in-rows and their triangles, the counts; then support, k, two
+		// frontiers and the ordering bitmap
+		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
+		if (in.nwords > 0xffffffffull || 16 * in.nwords + 20 * T + T / 8 + 16 * m + (uint64_t(1) << 20) > room)
+			break;
+		if ((rc = dalloc(c, &in.cells, in.nwords, "in-rows")) || (rc = dalloc(c, &in.live, m, "in-row counts")) ||
+			(rc = dalloc(c, &cnt, m, "in-row counts")) || (rc = dalloc(c, &sumsq, 1, "square sum")))
+			break;
+		if (cudaMemsetAsync(in.cells, 0, in.nwords * 16, c.stream) != cudaSuccess ||
+			cudaMemsetAsync(sumsq, 0, 8, c.stream) != cudaSuccess)
+		{
+			rc = fail(NUCLEUS34_E_CUDA, "memset");
+			break;
+		}
+		k_in_starts<<<gm, 256, 0, c.stream>>>(off, m, mats.erec);
+		k_in_set<<<gt, 256, 0, c.stream>>>(c.dtris, T, mats.erec, in.cells);
+		k_in_counts<<<gm, 256, 0, c.stream>>>(mats.erec, m, mats.cells, in.cells, width, cnt, in.live, sumsq);
+		c.launches += 3;
+		if ((rc = scan_u32(c, cnt, off, m)))
+			break;
+		if ((rc = dalloc(c, &in.tri, T, "in-row triangles")))
+			break;
+		k_in_firsts<<<gm, 256, 0, c.stream>>>(mats.erec, m, width, off, in.cells);
+		k_in_place<<<gt, 256, 0, c.stream>>>(c.dtris, T, mats.erec, in.cells, in.tri);
+		c.launches += 2;
+		uint64_t placed = 0;
+		if (cudaMemcpyAsync(&in.sum_te_sq, sumsq, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaMemcpyAsync(&placed, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaStreamSynchronize(c.stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
+		{
+			rc = fail(NUCLEUS34_E_CUDA, "in-row kernels");
+			break;
+		}
+		if (placed != T)
+			rc = fail(NUCLEUS34_E_CUDA, "internal: in-rows do not hold every triangle once");
+		*fits = true;
+	} while (false);
+	c.release(indeg);
+	c.release(width);
+	c.release(cnt);
+	c.release(off);
+	c.release(sumsq);
+	if (rc || !*fits)
+		free_in_rows(c, in);
+	return rc;
 }
 
-int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, uint64_t *total)
+void free_in_rows(Ctx &c, InMats &in)
+{
+	c.release(in.cells);
+	c.release(in.tri);
+	c.release(in.live);
+	in = InMats{};
+}
+
+int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total)
 {
 	unsigned long long *dtot = nullptr;
 	N34_TRY(dalloc(c, &dtot, 1, "support total"));
@@ -583,9 +618,8 @@ int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t
 		rc = fail(NUCLEUS34_E_CUDA, "memset");
 	if (!rc)
 	{
-		const uint32_t grid = grid_for(c, (c.T + 31) / 32, SUP_THREADS / 32, 32);
-		k_support_bits<<<grid, SUP_THREADS, 0, c.stream>>>(c.dtris, c.T, mats.erec, mats.cells, in.span, in.third,
-														   support, dtot);
+		k_support_bits<<<grid_for(c, c.T, SUP_THREADS, 32), SUP_THREADS, 0, c.stream>>>(
+			c.dtris, c.T, mats.erec, mats.cells, in.cells, in.live, support, dtot);
 		c.launches++;
 		if (cudaGetLastError() != cudaSuccess ||
 			cudaMemcpyAsync(&h, dtot, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
@@ -597,53 +631,30 @@ int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t
 	return rc;
 }
 
-int peel_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, int32_t *K, PeelCtl *hctl)
+int peel_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, int32_t *K, PeelCtl *hctl)
 {
-	const uint64_t T = c.T, words = (T + 31) / 32;
 	LoopBuffers b;
 	uint2 *crec = nullptr;
-	uint32_t *inbits = nullptr, *inlive = nullptr, *tpos = nullptr;
 	int rc = loop_alloc(c, b);
 	if (!rc)
-		rc = dalloc(c, &inbits, words, "in-list entry bits");
-	if (!rc)
-		rc = dalloc(c, &inlive, c.m, "in-list live counts");
-	if (!rc && cudaMemsetAsync(inbits, 0xff, words * 4, c.stream) != cudaSuccess)
-		rc = fail(NUCLEUS34_E_CUDA, "memset");
-	if (!rc)
 	{
-		k_in_lengths<<<grid_for(c, c.m, 256), 256, 0, c.stream>>>(in.span, c.m, inlive);
-		c.launches++;
-		// both optional: without room for them they are looked up
-		if (dalloc(c, &tpos, T, "in-list positions"))
-		{
-			tpos = nullptr;
-			clear_error();
-		}
-		else
-		{
-			k_in_positions<<<grid_for(c, T, 256), 256, 0, c.stream>>>(in.tri, T, tpos);
-			c.launches++;
-		}
-		if (dalloc(c, &crec, T, "c edge records"))
+		// optional: without room for it the records are looked up
+		if (dalloc(c, &crec, c.T, "c edge records"))
 		{
 			crec = nullptr;
 			clear_error();
 		}
 		else
 		{
-			k_c_records<<<grid_for(c, T, 256), 256, 0, c.stream>>>(c.dtris, T, mats.erec, crec);
+			k_c_records<<<grid_for(c, c.T, 256), 256, 0, c.stream>>>(c.dtris, c.T, mats.erec, crec);
 			c.launches++;
 		}
-		const BitPath path{c.dtris, c.dsrc, mats.erec, mats.cells, in.span, in.third, in.tri, inlive, inbits, tpos, crec};
+		const BitPath path{c.dtris, mats.erec, mats.cells, in.cells, in.tri, in.live, crec};
 		rc = run_peel_loop(c, b, path, support, K);
 	}
 	if (!rc)
 		rc = loop_finish(c, b, hctl);
 	c.release(crec);
-	c.release(tpos);
-	c.release(inbits);
-	c.release(inlive);
 	loop_release(c, b);
 	return rc;
 }

@@ -85,32 +85,6 @@ __global__ void k_inc_scatter(const uint32_t *__restrict__ tris, uint64_t T, con
 	}
 }
 
-// The same two passes for the in-lists: only the entry under c, with the
-// triangle's source as its third.
-__global__ void k_in_count(const uint32_t *__restrict__ tris, uint64_t T, uint32_t *__restrict__ cnt)
-{
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
-		atomicAdd(cnt + tris[3 * t + 2], 1u);
-}
-
-__global__ void k_in_scatter(const uint32_t *__restrict__ tris, uint64_t T, const uint32_t *__restrict__ src,
-							 const uint64_t *__restrict__ off, uint32_t *__restrict__ cursor, EntryStore keys,
-							 uint32_t *__restrict__ err)
-{
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
-	{
-		const uint32_t b = tris[3 * t + 1], e = tris[3 * t + 2];
-		const uint32_t s = atomicAdd(cursor + e, 1u);
-		// capacity guard: the counts pass sized every segment exactly
-		if (off[e] + s < off[e + 1])
-			keys.st(off[e] + s, (uint64_t(src[b]) << 32) | t);
-		else
-			atomicOr(err, 1u);
-	}
-}
-
 // Classifies edges by segment length into three work lists.
 __global__ void k_seg_classify(const uint64_t *__restrict__ incO, uint64_t m, uint32_t *__restrict__ lists,
 							   uint32_t *__restrict__ counts, uint64_t list_cap, unsigned long long *max_len)
@@ -321,29 +295,6 @@ __global__ void k_sum_sq(const uint64_t *__restrict__ off, uint64_t m, unsigned 
 		atomicAdd(out, acc);
 }
 
-// sum over edges of (triangles on the edge)^2 from the bit matrices and the
-// in-lists: an edge's symmetric row holds its triangles as a or b edge, its
-// in-list those as c edge.
-__global__ void k_sum_sq_bits(const uint2 *__restrict__ erec, const uint4 *__restrict__ cells,
-							  const uint64_t *__restrict__ off, uint64_t m, unsigned long long *__restrict__ out)
-{
-	unsigned long long acc = 0;
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
-	{
-		const uint2 r = erec[e];
-		unsigned long long d = off[e + 1] - off[e];
-		for (uint32_t q = 0; q < (r.y >> 16); ++q)
-			d += __popc(cells[r.x + q].z);
-		acc += d * d;
-	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		acc += __shfl_xor_sync(FULL, acc, o);
-	if (lane_id() == 0 && acc)
-		atomicAdd(out, acc);
-}
-
 // Splits the sorted keys into third[] and tri[]; with tpos, the key's slot
 // bits (30-31: which of the triangle's three entries) give tpos[3t + slot].
 __global__ void k_inc_split(const unsigned long long *__restrict__ keys, uint64_t n, uint32_t *__restrict__ third,
@@ -409,88 +360,6 @@ int sort_classes(Ctx &c, const uint32_t *lists, const uint32_t *counts, const ui
 }
 
 } // namespace
-
-int build_in_lists(Ctx &c, const BitMats &mats, Incidence &inc)
-{
-	const uint64_t T = c.T, m = c.m;
-	uint32_t *cnt = nullptr, *lists = nullptr, *counts = nullptr, *errf = nullptr;
-	unsigned long long *scratch = nullptr, *maxlen = nullptr, *sumsq = nullptr;
-	uint64_t *off = nullptr;
-	int rc = NUCLEUS34_OK;
-	do
-	{
-		if ((rc = dalloc(c, &off, m + 1, "in-list offsets")) || (rc = dalloc(c, &cnt, m, "in-list counts")) ||
-			(rc = dalloc(c, &errf, 1, "in-list check")) || (rc = dalloc(c, &counts, 4, "segment counts")) ||
-			(rc = dalloc(c, &maxlen, 1, "segment max")) || (rc = dalloc(c, &sumsq, 1, "segment square sum")))
-			break;
-		if (cudaMemsetAsync(cnt, 0, m * 4, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(errf, 0, 4, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(counts, 0, 16, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(maxlen, 0, 8, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(sumsq, 0, 8, c.stream) != cudaSuccess)
-		{
-			rc = fail(NUCLEUS34_E_CUDA, "memset");
-			break;
-		}
-		k_in_count<<<grid_for(c, T, 256), 256, 0, c.stream>>>(c.dtris, T, cnt);
-		c.launches++;
-		if ((rc = scan_u32(c, cnt, off, m)))
-			break;
-		if ((rc = dalloc(c, &inc.third, T, "in-list sources")) || (rc = dalloc(c, &inc.tri, T, "in-list triangles")))
-			break;
-		const EntryStore store{nullptr, inc.third, inc.tri};
-		if (cudaMemsetAsync(cnt, 0, m * 4, c.stream) != cudaSuccess)
-		{
-			rc = fail(NUCLEUS34_E_CUDA, "memset");
-			break;
-		}
-		k_in_scatter<<<grid_for(c, T, 256), 256, 0, c.stream>>>(c.dtris, T, c.dsrc, off, cnt, store, errf);
-		c.launches++;
-		c.release(cnt);
-		cnt = nullptr;
-		if ((rc = dalloc(c, &lists, 3 * m, "segment lists")))
-			break;
-		k_seg_classify<<<grid_for(c, m, 256), 256, 0, c.stream>>>(off, m, lists, counts, m, maxlen);
-		k_sum_sq_bits<<<grid_for(c, m, 256), 256, 0, c.stream>>>(mats.erec, mats.cells, off, m, sumsq);
-		c.launches += 2;
-		uint32_t hcounts[4] = {0, 0, 0, 0};
-		unsigned long long hmax = 0;
-		uint32_t herr = 0;
-		if (cudaMemcpyAsync(&inc.sum_te_sq, sumsq, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaMemcpyAsync(&herr, errf, 4, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaMemcpyAsync(hcounts, counts, 16, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaMemcpyAsync(&hmax, maxlen, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaStreamSynchronize(c.stream) != cudaSuccess)
-		{
-			rc = fail(NUCLEUS34_E_CUDA, "in-list classify");
-			break;
-		}
-		if (herr)
-		{
-			rc = fail(NUCLEUS34_E_CUDA, "internal: in-list segment overflow");
-			break;
-		}
-		if ((rc = sort_classes(c, lists, counts, hcounts, hmax, m, off, store, &scratch)))
-			break;
-		c.release(lists);
-		lists = nullptr;
-		if ((rc = dalloc(c, &inc.span, m, "in-list spans")))
-			break;
-		k_make_spans<<<grid_for(c, m, 256), 256, 0, c.stream>>>(off, m, inc.span);
-		c.launches++;
-		if (cudaGetLastError() != cudaSuccess)
-			rc = fail(NUCLEUS34_E_CUDA, "in-list kernels");
-	} while (false);
-	c.release(off);
-	c.release(cnt);
-	c.release(lists);
-	c.release(counts);
-	c.release(scratch);
-	c.release(maxlen);
-	c.release(errf);
-	c.release(sumsq);
-	return rc;
-}
 
 int build_incidence(Ctx &c, Incidence &inc, bool want_tpos, bool lean)
 {

@@ -43,13 +43,13 @@ struct DirectPath
 	// A warp takes a batch of consecutive frontier triangles; the entries of
 	// their clique lists are dealt out to the lanes across the batch.
 	__device__ __forceinline__ void debit(const LoopArgs &g, const uint32_t *F, uint32_t nF, uint32_t *Fn, PhaseSlot *slot,
-										  int32_t level, uint32_t) const
+										  int32_t level) const
 	{
 		extern __shared__ uint4 loop_smem[];
 		WarpMem &m = reinterpret_cast<WarpMem *>(loop_smem)[threadIdx.x >> 5];
 		Appender next{m.next, Fn, &slot->n, &g.ctl->c.error, g.T, 0u};
 		const uint32_t lane = lane_id();
-		const Units u = debit_units(nF, (gridDim.x * blockDim.x) >> 5);
+		const Units u = debit_units(nF, loop_warps());
 		claim_units(u.total, &slot->work, [&](uint32_t unit) {
 			const uint32_t stripe = unit & ((1u << u.shift) - 1u);
 			const uint32_t base = (unit >> u.shift) * u.ch;

@@ -3,8 +3,8 @@
 // All blocks of the launch are resident at once and run every round of the
 // peel, phases separated by grid barriers; nothing is launched and no size is
 // read by the host in between. A round is two phases:
-//   mark    the frontier's triangles get their k and their death stamp (the
-//           support word becomes 0x80000000 | round); the frontier before it
+//   mark    the frontier's triangles get their k and leave the scans (the
+//           support word becomes negative); the frontier before it
 //           is retired (what a path keeps per dead triangle is cleared)
 //   debit   every dying triangle enumerates its live four-cliques and debits
 //           the partners still alive; a partner that falls to the level is
@@ -95,15 +95,6 @@ __device__ __forceinline__ unsigned long long loop_ns()
 	unsigned long long t;
 	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
 	return t;
-}
-
-// A support word: weak load. Its sign and stamp only change in the mark phase;
-// debits of the running phase change the value of a live one alone.
-__device__ __forceinline__ int32_t ld_support(const int32_t *p)
-{
-	int32_t v;
-	asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
-	return v;
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
@@ -240,13 +231,9 @@ struct Appender
 };
 
 // Ownership of a clique among the members that die this round: the lowest id
-// (debit_partners' rule, cuNucleus34_ondemand.cu:237-276). True when dying
-// triangle t does not own it on account of a partner with support word s:
-// the partner died in an earlier round, or dies in this one with a lower id.
-__device__ __forceinline__ bool partner_blocks(int32_t s, uint32_t id, uint32_t t, uint32_t stamp)
-{
-	return s < 0 && (uint32_t(s) != stamp || id < t);
-}
+// (debit_partners' rule, cuNucleus34_ondemand.cu:237-276). Paths tell dying
+// members by flags of their own, set in the mark phase: a support word is never
+// read while other warps debit it.
 
 // How a debit phase is cut into units, which are claimed as the warps go:
 // batches of ch consecutive frontier triangles, at least sixteen per warp (a
@@ -539,7 +526,7 @@ __device__ __forceinline__ void order_write(const LoopArgs &g, uint32_t *__restr
 //   SMEM           bytes of dynamic shared memory per block
 //   mark(t)        a triangle begins to die
 //   retire(t)      it died in the round before
-//   debit(g, F, nF, Fn, slot, level, stamp)  the debit phase (all threads call)
+//   debit(g, F, nF, Fn, slot, level)  the debit phase (all threads call)
 template <class Path>
 __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path path)
 {
@@ -591,12 +578,11 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 			nF = n;
 			lap(2);
 		}
-		const uint32_t stamp = 0x80000000u | round;
 		block_shares(uint64_t(nF) + nPrev, [&](uint64_t i) {
 			if (i < nF)
 			{
 				const uint32_t t = F[i];
-				g.S[t] = int32_t(stamp);
+				g.S[t] = -1;
 				g.K[t] = int32_t(level);
 				if (g.R)
 					g.R[t] = round;
@@ -608,7 +594,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 		if (!(ok = phase_end(g.ctl, phase, n, mn, false)))
 			break;
 		lap(0);
-		path.debit(g, F, nF, Fp, &g.ctl->slot[phase & 3], int32_t(level), stamp);
+		path.debit(g, F, nF, Fp, &g.ctl->slot[phase & 3], int32_t(level));
 		if (!(ok = phase_end(g.ctl, phase, n, mn, false)))
 			break;
 		lap(1);

@@ -40,9 +40,22 @@ struct BitMats
 	// w: symmetric, zero at first; the peel sets both when it begins to die.
 	// One 16-byte load tells a triangle's id and state.
 	uint4 *cells = nullptr;
-	// per oriented edge: {first cell of its row, W << 16 | its position in N+(u)}
-	uint2 *erec = nullptr;
+	// per oriented edge: {first cell of its row, W << 16 | its position in
+	// N+(u), first cell of its in-row, its column among its head's in-edges}
+	uint4 *erec = nullptr;
 	uint64_t nwords = 0;
+};
+
+// The same for the triangles that lie on an edge as its c edge. Edge u -> v has
+// an in-row of ceil(in-degree of u / 32) cells over u's in-edges y -> u (in any
+// order): a bit is the triangle (y, u, v).
+struct InMats
+{
+	uint4 *cells = nullptr; // as above, y counting positions in tri
+	uint32_t *tri = nullptr; // triangle ids, in-row by in-row
+	uint2 *live = nullptr;  // per oriented edge: {triangles of its in-row not dead, cells of the in-row}
+	uint64_t nwords = 0;
+	unsigned long long sum_te_sq = 0; // sum over edges of (triangles on the edge)^2
 };
 
 // Triangle -> four-clique incidence of the direct variant.
@@ -63,9 +76,6 @@ void free_mats(Ctx &c, BitMats &mats);
 // lean: no 64-bit key array (entries sorted in place as pairs) and no tpos.
 int build_incidence(Ctx &c, Incidence &inc, bool want_tpos, bool lean = false);
 void free_incidence(Ctx &c, Incidence &inc);
-// The in-lists of the bit-matrix form: only the entry under each triangle's c
-// edge (third = its source), so T entries; inc.span/third/tri as above.
-int build_in_lists(Ctx &c, const BitMats &mats, Incidence &inc);
 // Sorts every segment [off[s], off[s+1]) of keys ascending (incidence.cu's
 // segmented sort; nseg < 2^32).
 int sort_segments_u64(Ctx &c, unsigned long long *keys, const uint64_t *off, uint64_t nseg);
@@ -86,9 +96,12 @@ int segments_after_support(Ctx &c, const int32_t *support);
 int segments_after_peel(Ctx &c);
 // The bit-matrix form of the support count and the peel (on-demand variant).
 bool bit_form_wanted(const Ctx &c, int variant);
-bool bit_form_fits(const Ctx &c, const BitMats &mats);
-int count_support_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, uint64_t *total);
-int peel_bits(Ctx &c, const BitMats &mats, const Incidence &in, int32_t *support, int32_t *K, PeelCtl *hctl);
+// Builds the in-rows; *fits is false, and nothing is left, when they and what
+// the form needs beside them exceed the room left.
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits);
+void free_in_rows(Ctx &c, InMats &in);
+int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total);
+int peel_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, int32_t *K, PeelCtl *hctl);
 // The direct variant's peel over the clique list.
 int peel_direct(Ctx &c, const CliqueCsr &csr, int32_t *support, int32_t *K, PeelCtl *hctl);
 // Device-resident peel of the on-demand variant's list form; K receives the final k of every triangle.

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__rest
 														  const uint32_t *__restrict__ src, uint64_t j0, uint64_t j1,
 														  const uint64_t *__restrict__ woff, uint64_t wbase,
 														  const uint64_t *__restrict__ aoff, uint4 *__restrict__ cells,
-														  const uint32_t *__restrict__ cols, uint2 *__restrict__ erec)
+														  const uint32_t *__restrict__ cols, uint4 *__restrict__ erec)
 {
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t j = j0 + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < j1; j += stride)
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__rest
 			cells[base + q] = c;
 		}
 		if (erec)
-			erec[j] = make_uint2(uint32_t(base), (W << 16) | ia);
+			erec[j] = make_uint4(uint32_t(base), (W << 16) | ia, 0u, 0u);
 	}
 }
 
@@ -438,8 +438,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 	const uint64_t n = c.n, m = c.m;
 	uint64_t *words = nullptr, *woff = nullptr, *aoff = nullptr;
 	uint32_t *rowcnt = nullptr, *cols = nullptr, *err = nullptr;
-	uint4 *cells = nullptr;
-	uint2 *erec = nullptr;
+	uint4 *cells = nullptr, *erec = nullptr;
 	int rc = NUCLEUS34_OK;
 	auto cleanup = [&] {
 		c.release(words);
