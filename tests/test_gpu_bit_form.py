@@ -49,6 +49,21 @@ def test_frontier_order_and_claims(n34, oracle, case, shift):
         assert r["four_clique_count"] == o.Q and r["k_max"] == o.k_max and r["k_avg"] == o.k_avg
 
 
+# frontiers put in id order: graphs of 2^24 triangles and more, with the
+# threshold at its lowest, at its default and off
+def test_ordered_frontiers_match_the_list_form(n34):
+    g = n34.graph_from_edges(*n34.gen_rgg(200003, 32, 9))
+    want = n34.decompose(g, variant="ondemand", flags=n34.OPT_LEAN_MEMORY)
+    assert want.result["triangle_count"] >= 2 ** 24
+    with n34.Context() as ctx:
+        ctx.upload(g)
+        for shift in (31, 12, 0xffffffff):
+            ctx.set_tune({"sort_shift": shift})
+            r = ctx.run("ondemand")
+            assert r["peeling_iterations"] == want.result["peeling_iterations"]
+            assert np.array_equal(ctx.copy_k(r["triangle_count"]), want.k)
+
+
 # an acyclic orientation that is not by degree: every source's list is long
 @pytest.mark.parametrize("seed", [1, 2])
 def test_other_orientations(n34, seed):
