@@ -343,10 +343,10 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 			break;
 		}
 		c.lean_run = false;
-		// the on-demand variant runs on the listing's bit matrices when they
-		// were kept and the rest fits beside them, else on the incidence lists
+		// both variants run on the listing's bit matrices when they were kept and
+		// the rest fits beside them, else on the incidence lists
 		bool bits = c.T && mats.cells;
-		if (bits && (rc = build_in_rows(c, mats, in, &bits)))
+		if (bits && (rc = build_in_rows(c, mats, in, variant == NUCLEUS34_DIRECT, &bits)))
 			break;
 		if (!bits)
 			free_mats(c, mats);
@@ -380,7 +380,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (variant == NUCLEUS34_DIRECT && (rc = dalloc(c, &own, c.T, "clique owner counts")))
 				break;
-			if ((rc = bits ? count_support_bits(c, mats, in, S, &total) : count_support(c, inc, S, &total, own)))
+			if ((rc = bits ? count_support_bits(c, mats, in, S, &total, own) : count_support(c, inc, S, &total, own)))
 				break;
 			if (total % 4)
 			{
@@ -394,7 +394,28 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 		N34_CUDA(cudaEventRecord(ev.e[3], c.stream));
 		if (variant == NUCLEUS34_DIRECT && total)
 		{
-			if ((rc = list_cliques(c, inc, S, own, csr)))
+			rc = bits ? list_cliques_bits(c, mats, in, S, own, csr) : list_cliques(c, inc, S, own, csr);
+			if (bits && rc == NUCLEUS34_E_OOM_BUDGET)
+			{
+				// the incidence lists may be smaller than the rows
+				clear_error();
+				bits = false;
+				free_mats(c, mats);
+				free_in_rows(c, in);
+				free_clique_csr(c, csr);
+				c.release(c.dquds);
+				c.dquds = nullptr;
+				c.release(own);
+				c.release(S);
+				own = nullptr;
+				S = nullptr;
+				if ((rc = build_incidence(c, inc, false, false)) || (rc = dalloc(c, &S, c.T, "support")) ||
+					(rc = dalloc(c, &own, c.T, "clique owner counts")) ||
+					(rc = count_support(c, inc, S, &total, own)))
+					break;
+				rc = list_cliques(c, inc, S, own, csr);
+			}
+			if (rc)
 				break;
 			if (c.Q != total / 4)
 			{
@@ -429,9 +450,9 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 				break;
 			if (total)
 			{
-				rc = variant == NUCLEUS34_DIRECT ? peel_direct(c, csr, S, c.dK, &pc)
-					 : bits						 ? peel_bits(c, mats, in, S, c.dK, &pc)
-												 : peel(c, inc, S, c.dK, &pc);
+				rc = csr.off ? peel_direct(c, csr, S, c.dK, &pc)
+					 : bits	 ? peel_bits(c, mats, in, S, c.dK, &pc)
+							 : peel(c, inc, S, c.dK, &pc);
 				if (rc)
 					break;
 				peeled = true;

@@ -1,4 +1,5 @@
-// The on-demand variant on bit matrices: four-clique support and peel.
+// The peel on bit matrices, and the in-rows that it and the support count
+// (bitcliques.cu) share.
 //
 // Reference: count_support and debit_partners (nucleus/cuNucleus34_ondemand.cu:
 // 176-194, 203-305) find a triangle's cliques by a 3-way zipper over the
@@ -42,8 +43,6 @@ namespace n34 {
 
 namespace {
 
-constexpr int SUP_THREADS = 256;
-
 // ---- in-rows -----------------------------------------------------------------
 
 // column of every edge among its head's in-edges, and the in-degrees
@@ -53,6 +52,28 @@ __global__ void k_in_columns(const uint32_t *__restrict__ E, uint64_t m, uint32_
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
 		erec[e].w = atomicAdd(indeg + E[e], 1u);
+}
+
+// key of every in-edge at its place among its head's (any order)
+__global__ void k_in_keys(const uint32_t *__restrict__ E, const uint32_t *__restrict__ src, uint64_t m,
+						  const uint64_t *__restrict__ in_off, const uint4 *__restrict__ erec,
+						  unsigned long long *__restrict__ keys)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
+		keys[in_off[E[e]] + erec[e].w] = (unsigned long long)src[e] << 32 | e;
+}
+
+// columns in the order of the sorted keys
+__global__ void k_in_sorted_columns(const uint32_t *__restrict__ E, const unsigned long long *__restrict__ keys,
+									uint64_t m, const uint64_t *__restrict__ in_off, uint4 *__restrict__ erec)
+{
+	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+	for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride)
+	{
+		const uint32_t e = uint32_t(keys[i]);
+		erec[e].w = uint32_t(i - in_off[E[e]]);
+	}
 }
 
 // cells of every edge's in-row
@@ -156,39 +177,6 @@ __global__ void k_in_place(const uint32_t *__restrict__ tris, uint64_t T, const 
 		const uint2 c = __ldg(reinterpret_cast<const uint2 *>(cells + row + (col >> 5)));
 		tri[c.y + __popc(c.x & ((1u << (col & 31)) - 1u))] = uint32_t(t);
 	}
-}
-
-// ---- support -------------------------------------------------------------------
-
-// support[t] = cliques on t: the common bits of its two rows and of its two
-// in-rows, one thread per triangle (neighbours share their source, so the rows
-// come from L1).
-__global__ void __launch_bounds__(SUP_THREADS) k_support_bits(
-	const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
-	const uint4 *__restrict__ in_rows, const uint2 *__restrict__ in_live, int32_t *__restrict__ support,
-	unsigned long long *__restrict__ total)
-{
-	unsigned long long acc = 0;
-	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
-	{
-		const uint32_t a = __ldg(tris + 3 * t), b = __ldg(tris + 3 * t + 1);
-		const uint4 ra = __ldg(erec + a), rb = __ldg(erec + b);
-		const uint2 la = __ldg(in_live + a), lb = __ldg(in_live + b);
-		uint32_t cnt = 0;
-		for (uint32_t q = 0; q < (ra.y >> 16); ++q)
-			cnt += __popc(__ldg(&rows[ra.x + q].z) & __ldg(&rows[rb.x + q].z));
-		if (la.x && lb.x)
-			for (uint32_t q = 0; q < la.y; ++q)
-				cnt += __popc(__ldg(&in_rows[ra.z + q].x) & __ldg(&in_rows[rb.z + q].x));
-		support[t] = int32_t(cnt);
-		acc += cnt;
-	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		acc += __shfl_xor_sync(FULL, acc, o);
-	if (lane_id() == 0 && acc)
-		atomicAdd(total, acc);
 }
 
 // ---- peel ----------------------------------------------------------------------
@@ -514,18 +502,18 @@ struct BitPath
 
 } // namespace
 
-// The bit form serves the on-demand variant unless a flag asks for one of the
-// list forms (a layout, an owner test or a schedule of theirs).
+// The bit form serves the direct variant, and the on-demand variant unless a
+// flag asks for the list form (a layout, an owner test or a schedule of it).
 bool bit_form_wanted(const Ctx &c, int variant)
 {
 	constexpr uint32_t LIST_FORM = NUCLEUS34_OPT_STAMP_PEEL | NUCLEUS34_OPT_LEAN_MEMORY | NUCLEUS34_OPT_HOST_LOOP |
 								   NUCLEUS34_OPT_NO_SMALL_ROUNDS | NUCLEUS34_OPT_FRONTIER_BY_C |
 								   NUCLEUS34_OPT_CHUNKED_DEBIT | NUCLEUS34_OPT_SCALAR_SCANS |
 								   NUCLEUS34_OPT_PIPELINED_DEBIT | NUCLEUS34_OPT_DEBIT_CURSOR;
-	return variant == NUCLEUS34_ONDEMAND && !(c.opt_flags & LIST_FORM);
+	return variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM);
 }
 
-int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits)
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits)
 {
 	const uint64_t T = c.T, m = c.m;
 	*fits = false;
@@ -547,6 +535,17 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits)
 		k_in_columns<<<gm, 256, 0, c.stream>>>(c.dE, m, indeg, mats.erec);
 		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dsrc, m, indeg, width);
 		c.launches += 2;
+		if (by_source)
+		{
+			if ((rc = dalloc(c, &in.in_off, c.n + 1, "in-edge offsets")) || (rc = scan_u32(c, indeg, in.in_off, c.n)) ||
+				(rc = dalloc(c, &in.in_edges, m, "in-edges")))
+				break;
+			k_in_keys<<<gm, 256, 0, c.stream>>>(c.dE, c.dsrc, m, in.in_off, mats.erec, in.in_edges);
+			if ((rc = sort_segments_u64(c, in.in_edges, in.in_off, c.n)))
+				break;
+			k_in_sorted_columns<<<gm, 256, 0, c.stream>>>(c.dE, in.in_edges, m, in.in_off, mats.erec);
+			c.launches += 2;
+		}
 		c.release(indeg);
 		indeg = nullptr;
 		if ((rc = scan_u32(c, width, off, m)))
@@ -601,6 +600,12 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits)
 	c.release(sumsq);
 	if (rc || !*fits)
 		free_in_rows(c, in);
+	if (rc == NUCLEUS34_E_OOM_BUDGET)
+	{
+		clear_error();
+		*fits = false;
+		return NUCLEUS34_OK;
+	}
 	return rc;
 }
 
@@ -609,30 +614,9 @@ void free_in_rows(Ctx &c, InMats &in)
 	c.release(in.cells);
 	c.release(in.tri);
 	c.release(in.live);
+	c.release(in.in_edges);
+	c.release(in.in_off);
 	in = InMats{};
-}
-
-int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total)
-{
-	unsigned long long *dtot = nullptr;
-	N34_TRY(dalloc(c, &dtot, 1, "support total"));
-	unsigned long long h = 0;
-	int rc = NUCLEUS34_OK;
-	if (cudaMemsetAsync(dtot, 0, 8, c.stream) != cudaSuccess)
-		rc = fail(NUCLEUS34_E_CUDA, "memset");
-	if (!rc)
-	{
-		k_support_bits<<<grid_for(c, c.T, SUP_THREADS, 32), SUP_THREADS, 0, c.stream>>>(
-			c.dtris, c.T, mats.erec, mats.cells, in.cells, in.live, support, dtot);
-		c.launches++;
-		if (cudaGetLastError() != cudaSuccess ||
-			cudaMemcpyAsync(&h, dtot, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaStreamSynchronize(c.stream) != cudaSuccess)
-			rc = fail(NUCLEUS34_E_CUDA, "support count");
-	}
-	c.release(dtot);
-	*total = h;
-	return rc;
 }
 
 int peel_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, int32_t *K, PeelCtl *hctl)

@@ -48,7 +48,7 @@ struct BitMats
 
 // The same for the triangles that lie on an edge as its c edge. Edge u -> v has
 // an in-row of ceil(in-degree of u / 32) cells over u's in-edges y -> u (in any
-// order): a bit is the triangle (y, u, v).
+// order, or by y: see build_in_rows): a bit is the triangle (y, u, v).
 struct InMats
 {
 	uint4 *cells = nullptr; // as above, y counting positions in tri
@@ -56,6 +56,10 @@ struct InMats
 	uint2 *live = nullptr;  // per oriented edge: {triangles of its in-row not dead, cells of the in-row}
 	uint64_t nwords = 0;
 	unsigned long long sum_te_sq = 0; // sum over edges of (triangles on the edge)^2
+	// with by_source only (the direct variant's clique list): every vertex's
+	// in-edges as y << 32 | edge, ascending, and where they start
+	unsigned long long *in_edges = nullptr; // m
+	uint64_t *in_off = nullptr;             // n + 1
 };
 
 // Triangle -> four-clique incidence of the direct variant.
@@ -94,13 +98,20 @@ void free_clique_csr(Ctx &c, CliqueCsr &csr);
 int segments_after_listing(Ctx &c);
 int segments_after_support(Ctx &c, const int32_t *support);
 int segments_after_peel(Ctx &c);
-// The bit-matrix form of the support count and the peel (on-demand variant).
+// The bit-matrix form of the support count, the clique list and the peel.
 bool bit_form_wanted(const Ctx &c, int variant);
 // Builds the in-rows; *fits is false, and nothing is left, when they and what
-// the form needs beside them exceed the room left.
-int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool *fits);
+// the form needs beside them exceed the room left. by_source: columns ascend
+// with the in-edge's source.
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits);
 void free_in_rows(Ctx &c, InMats &in);
-int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total);
+// own (optional, needs by_source): cliques whose lowest triangle is t.
+int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total,
+					   uint32_t *own);
+// Direct variant: the clique list and, where the peel uses them in place of the
+// rows (which it then gives back), the triangle -> clique lists.
+int list_cliques_bits(Ctx &c, BitMats &mats, InMats &in, const int32_t *support, const uint32_t *own,
+					  CliqueCsr &csr);
 int peel_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, int32_t *K, PeelCtl *hctl);
 // The direct variant's peel over the clique list.
 int peel_direct(Ctx &c, const CliqueCsr &csr, int32_t *support, int32_t *K, PeelCtl *hctl);
