@@ -190,6 +190,13 @@ __global__ void k_c_records(const uint32_t *__restrict__ tris, uint64_t T, const
 		crec[t] = __ldg(reinterpret_cast<const uint2 *>(erec + __ldg(tris + 3 * t + 2)));
 }
 
+// LIVE: counts of the live triangles of every in-row follow the peel, so that
+// in-rows without any are passed by. Of use where in-rows are long (R-MAT scale
+// 18, 8 words a row: peel 170 ms with them, 178 without; scale 16: 32.1 and
+// 33.6); where they are two words or less, a word costs no more than its count
+// (geometric graphs of 1.1e8 and 4.5e7 triangles: 52.8 and 22.9 ms with the
+// counts, 50.9 and 22.4 without).
+template <bool LIVE>
 struct BitPath
 {
 	const uint32_t *tris;
@@ -220,7 +227,8 @@ struct BitPath
 		atomicAnd(&cells[ra.x + (j >> 5)].z, ~(1u << (j & 31)));
 		atomicAnd(&cells[rb.x + (p >> 5)].z, ~(1u << (p & 31)));
 		atomicAnd(&in_cells[in + (col >> 5)].z, ~(1u << (col & 31)));
-		atomicSub(&in_live[c].x, 1u);
+		if (LIVE)
+			atomicSub(&in_live[c].x, 1u);
 	}
 
 	__device__ __forceinline__ uint2 row_of(uint32_t e) const
@@ -434,7 +442,7 @@ struct BitPath
 				const uint4 ra = __ldg(erec + a), rb = __ldg(erec + b);
 				// none live under one of the edges: no clique through the in-rows
 				const uint2 lb = in_live[b];
-				const uint32_t na = in_live[a].x, nc = in_live[c].x;
+				const uint32_t na = LIVE ? in_live[a].x : 1u, nc = LIVE ? in_live[c].x : 1u;
 				row_w = ra.x;
 				row_v = rb.x;
 				W = do_rows ? ra.y >> 16 : 0u;
@@ -637,8 +645,12 @@ int peel_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, i
 			k_c_records<<<grid_for(c, c.T, 256), 256, 0, c.stream>>>(c.dtris, c.T, mats.erec, crec);
 			c.launches++;
 		}
-		const BitPath path{c.dtris, mats.erec, mats.cells, in.cells, in.tri, in.live, crec};
-		rc = run_peel_loop(c, b, path, support, K);
+		if (in.nwords > 2 * c.m)
+			rc = run_peel_loop(c, b, BitPath<true>{c.dtris, mats.erec, mats.cells, in.cells, in.tri, in.live, crec},
+							   support, K);
+		else
+			rc = run_peel_loop(c, b, BitPath<false>{c.dtris, mats.erec, mats.cells, in.cells, in.tri, in.live, crec},
+							   support, K);
 	}
 	if (!rc)
 		rc = loop_finish(c, b, hctl);

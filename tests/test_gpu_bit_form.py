@@ -105,3 +105,17 @@ def test_rounds_and_work_measure_match_the_list_form(n34):
     b = n34.decompose(g, variant="ondemand", flags=n34.OPT_LEAN_MEMORY).result
     for key in ("peeling_iterations", "sum_te_sq", "four_clique_count", "k_max"):
         assert a[key] == b[key], key
+
+
+# in-rows on both sides of two words per edge (with and without live counts)
+@pytest.mark.parametrize("hubs", [1, 40, 200])
+def test_in_row_widths(n34, oracle, hubs):
+    n, rng = 400, np.random.default_rng(hubs)
+    hub = np.arange(hubs, dtype=np.uint32) + n
+    i, j = dense(n, 0.08, hubs)
+    k = rng.random((n, hubs)) < 0.5
+    s = np.concatenate([i, np.repeat(np.arange(n, dtype=np.uint32), hubs)[k.ravel()]])
+    t = np.concatenate([j, np.tile(hub, n)[k.ravel()]])
+    a, b = dense(hubs, 0.5, 3, offset=n)
+    g = n34.graph_from_edges(np.concatenate([s, a]), np.concatenate([t, b]))
+    same_as_oracle(n34.decompose(g, variant="ondemand"), oracle.decompose(g, quds_cap=0))
