@@ -67,7 +67,7 @@ def parse():
     p.add_argument("--capture-run", action="store_true",
                    help="exactly one decomposition of the workload graph (for ncu captures); prints its record")
     p.add_argument("--peel-profile", action="store_true",
-                   help="with --capture-run: per-step profiling mode (plain launches, per-round trace on stderr)")
+                   help="with --capture-run: profiling mode (time per phase kind of the peel on stderr)")
     p.add_argument("--host-loop", action="store_true",
                    help="with --capture-run: the peel's host-driven replay graphs instead of the device loop")
     p.add_argument("--batch-graphs", type=int, default=4096)
@@ -712,8 +712,8 @@ def main():
     launches = sum(r["gpu_launches"] for r in results)
     ctx.close()
 
-    # ---- one untimed run with per-kernel CUDA events in the peel: device time
-    # of the re-enumeration (debit) kernels for the roofline ----
+    # ---- one untimed run whose peel reports the time of its debit phases, for
+    # the roofline ----
     with n34.Context(device=device, flags=n34.OPT_PROFILE_PEEL) as pctx:
         pctx.upload(g)
         prof = pctx.run(a.variant)
@@ -798,17 +798,6 @@ def main():
     return 0
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic
-# byte of k_support, from its single-launch ncu capture on a smaller case of
-# the same workload (R-MAT scale 17), applied to this run's algorithmic bytes:
-# its traffic grows with the lists it reads. The debit runs as thousands of
-# launches of different sizes, and an ncu capture covers one to three of them,
-# so no per-launch figure of its traffic matches the whole-peel `achieved`:
-# its `traffic` is null, and its single-round captures are summarised beside
-# the kernel's profile.
-NCU_TRAFFIC_PER_ALG_BYTE = {"k_support": 0.028}
-
-
 def roofline(r, prof, peaks, kind):
     """HBM roofline of the two intersection phases.
 
@@ -817,26 +806,24 @@ def roofline(r, prof, peaks, kind):
     triangle reads its three edges' incidence lists (4 B per entry), its own
     record and list bounds (36 B), and each of the 4Q clique occurrences reads
     3 partner ids (48 B per clique). The support count performs one
-    enumeration in one launch (k_support); the peel performs it once more,
-    spread over its rounds (k_debit_flags_warp + k_debit_flags_thread, two
-    launches per round), timed by CUDA events around those kernels in a
-    separate profiling run of the same workload. Both kernels intersect only
-    the two shortest lists of a triangle, so they move fewer bytes than this
-    bound and a fraction above 1 is possible."""
+    enumeration in one launch (k_support_bits); the peel performs it once more,
+    spread over the debit phases of its one launch (k_peel_loop), which the
+    kernel times itself in a separate run of the same workload. Both read bit
+    rows in place of lists (32 candidates per 16 bytes), so they move far fewer
+    bytes than this bound and a fraction above 1 is possible. traffic is null:
+    no capture of these kernels at this size was taken."""
     T, Q, S2 = r["triangle_count"], r["four_clique_count"], r["sum_te_sq"]
     alg = 4 * S2 + 36 * T + 48 * Q
     peak = peaks.get("hbm_gbs")
     pk = f"{kind} ({'hbm_gbs' if kind == 'measured' else 'fallback 6.65 TB/s'})"
     out = []
-    for name, key, t, launches, what in (
-            ("k_debit_flags_warp+k_debit_flags_thread", "debit", prof.get("t_peel_debit", 0.0),
-             2 * int(prof.get("peeling_iterations", 0)), "peel re-enumeration, all rounds (profiling run)"),
-            ("k_support", "k_support", r["t_support"], 1, "support count (one launch, timed run)")):
+    for name, t, launches, what in (
+            ("k_peel_loop", prof.get("t_peel_debit", 0.0), 1, "debit phases of the peel, all rounds (profiling run)"),
+            ("k_support_bits", r["t_support"], 1, "support count (one launch, timed run)")):
         ach = alg / t / 1e9 if t > 0 else None
-        ratio = NCU_TRAFFIC_PER_ALG_BYTE.get(key)
         out.append({"kernel": name, "what": what, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                     "frac": (ach / peak) if (ach and peak) else None,
-                    "traffic": (ratio * alg) if ratio else None, "algorithmic_bytes": alg,
+                    "traffic": None, "algorithmic_bytes": alg,
                     "device_seconds": t, "launches": launches, "peak_kind": pk,
                     "definition": "4*sum_e T(e)^2 + 36T + 48Q bytes per full enumeration (zipper bound)"})
     # the dominant kernel is the one with the larger device time

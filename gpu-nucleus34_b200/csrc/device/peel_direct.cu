@@ -12,9 +12,10 @@
 // to die and left set) tells apart: no support is read beside the atomics.
 //
 // As launches (11 per round, half of them empty) a round took 34 us on R-MAT
-// scale 14 and 55 us on the geometric graph with 50k points; here 19 and 28.
+// scale 14 and 55 us on the geometric graph with 50k points; here 16.5 and 25.
 // The clique ids and members of a round stream from L2 or memory (R-MAT scale
-// 14 holds 1.1 GB of them); the atomics and the barriers are the rest.
+// 14 holds 1.1 GB of them, and takes the rows instead: see list_cliques_bits);
+// the atomics and the barriers are the rest.
 #include "pipeline.cuh"
 
 #include "peel_loop.cuh"

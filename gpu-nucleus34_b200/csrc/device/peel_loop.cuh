@@ -17,7 +17,7 @@
 // Round-to-round cost is what bounds the small graphs and the long tails of
 // the large ones: with every step of a round a kernel of its own (13 launches
 // in a CUDA graph's while node) a round took 38 us on R-MAT scale 12 and 66 us
-// on scale 16, with most of the launches empty; here it takes 13 and 33 us, of
+// on scale 16, with most of the launches empty; here it takes 11.5 and 28 us, of
 // which a barrier is 1.4.
 //
 // The counters that a phase fills (appended triangles, minimum support) live

@@ -84,8 +84,8 @@ typedef struct
  * as plain launches with CUDA events around every step (slower). */
 #define NUCLEUS34_OPT_PROFILE_PEEL 0x2u
 /* The on-demand variant peels on the triangle listing's bit matrices, all
- * rounds in one cooperative launch, as the direct variant does on its clique
- * list. Its list form, on the incidence lists, serves graphs whose matrices do
+ * rounds in one cooperative launch; so does the direct variant, on its clique
+ * list up to 2^24 cliques. The list form, on the incidence lists, serves graphs whose matrices do
  * not fit in the memory budget, and the flags below that select a layout or a
  * schedule of it (STAMP_PEEL, LEAN_MEMORY, HOST_LOOP, NO_SMALL_ROUNDS,
  * FRONTIER_BY_C, CHUNKED_DEBIT, SCALAR_SCANS, PIPELINED_DEBIT, DEBIT_CURSOR;
