@@ -1,5 +1,6 @@
 // Four-clique support per triangle, and the direct variant's clique list and
-// triangle -> clique CSR.
+// triangle -> clique CSR, on incidence lists (where the bit rows of
+// bitcliques.cu are not used).
 //
 // Reference: count_support (nucleus/cuNucleus34_ondemand.cu:176-194) counts
 // cliques per triangle through the 3-way zipper; the direct program lists the
