@@ -27,9 +27,10 @@
 //               of the word below ib. No search is needed for c.
 // The matrices can be kept (BitMats) for the on-demand variant's support count
 // and peel (bitpeel.cu).
-// Steps 1-2 hold 20 bytes per (column, row tile) of each source; when
+// Steps 1-2 hold 12 bytes per (column, row tile) of each source; when
 // those do not fit the budget the sources are taken in chunks, counting all
-// of them first and repeating steps 1-2 before each chunk's writes.
+// of them first and repeating steps 1-2 before each chunk's writes. The kept
+// form takes 16 bytes per tile more, and is left out where these do not fit.
 //
 // The pair-test kernels below (every (ia, ib) tested by a binary search of w
 // in N+(v)) serve callers that manage their own memory and cannot give the
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_cols(const uint32_t *__res
 __global__ void __launch_bounds__(TRI_THREADS) k_list_rows(const uint32_t *__restrict__ O, uint64_t u0, uint64_t u1,
 														   const uint64_t *__restrict__ woff, uint64_t wbase,
 														   const uint32_t *__restrict__ cols,
-														   uint4 *__restrict__ cells, uint32_t *__restrict__ rowcnt)
+														   uint2 *__restrict__ rows, uint32_t *__restrict__ rowcnt)
 {
 	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 	const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_rows(const uint32_t *__res
 						rw = b;
 				}
 				if (row < d)
-					cells[base + uint64_t(row) * W + q] = make_uint4(rw, tot, 0u, 0u);
+					rows[base + uint64_t(row) * W + q] = make_uint2(rw, tot);
 				tot += __popc(rw);
 			}
 			if (row < d)
@@ -321,17 +322,18 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_rows(const uint32_t *__res
 	}
 }
 
-// Step 3: canonical ids in the cells. One thread per edge a in [j0, j1): the
+// Step 3: canonical ids in the rows. One thread per edge a in [j0, j1): the
 // prefix of each of its words becomes the id of the word's first triangle
-// (T < 2^32 was checked). With erec, the column word beside it makes the cell's
-// symmetric word (triangles of u that hold vertex ia and vertex 32q + i,
-// whichever of the two is the head), and the edge's record gets its row and its
-// position.
+// (T < 2^32 was checked). With cells, the word and its id go there instead,
+// the column word beside it makes the cell's symmetric word (triangles of u
+// that hold vertex ia and vertex 32q + i, whichever of the two is the head), and
+// the edge's record gets its row and its position.
 __global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__restrict__ O,
 														  const uint32_t *__restrict__ src, uint64_t j0, uint64_t j1,
 														  const uint64_t *__restrict__ woff, uint64_t wbase,
-														  const uint64_t *__restrict__ aoff, uint4 *__restrict__ cells,
-														  const uint32_t *__restrict__ cols, uint4 *__restrict__ erec)
+														  const uint64_t *__restrict__ aoff, uint2 *__restrict__ rows,
+														  const uint32_t *__restrict__ cols, uint4 *__restrict__ cells,
+														  uint4 *__restrict__ erec)
 {
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t j = j0 + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < j1; j += stride)
@@ -342,11 +344,11 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__rest
 		const uint32_t first = uint32_t(aoff[j]);
 		for (uint32_t q = 0; q < W; ++q)
 		{
-			uint4 c = cells[base + q];
-			c.y += first;
-			if (erec)
-				c.z = c.x | __ldg(cols + base + q);
-			cells[base + q] = c;
+			const uint2 r = rows[base + q];
+			if (cells)
+				cells[base + q] = make_uint4(r.x, r.y + first, r.x | __ldg(cols + base + q), 0u);
+			else
+				rows[base + q].y = r.y + first;
 		}
 		if (erec)
 			erec[j] = make_uint4(uint32_t(base), (W << 16) | ia, 0u, 0u);
@@ -354,12 +356,14 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_ids(const uint32_t *__rest
 }
 
 // Step 4: the triangles at their canonical positions. One warp per oriented
-// edge b in [j0, j1), the merge of step 1 again.
+// edge b in [j0, j1), the merge of step 1 again. STEP: a row word and its id
+// are the first 8 of every 8 * STEP bytes (1: the rows, 2: the cells).
+template <uint32_t STEP>
 __global__ void __launch_bounds__(TRI_THREADS) k_list_write(const uint32_t *__restrict__ O,
 															const uint32_t *__restrict__ E,
 															const uint32_t *__restrict__ src, uint64_t j0,
 															uint64_t j1, const uint64_t *__restrict__ woff,
-															uint64_t wbase, const uint4 *__restrict__ cells, uint64_t T,
+															uint64_t wbase, const uint2 *__restrict__ rows, uint64_t T,
 															uint32_t *__restrict__ tris, uint32_t *__restrict__ err)
 {
 	const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(TRI_THREADS) k_list_write(const uint32_t *__re
 			if (!found)
 				return;
 			const uint32_t ia = (k << 5) + lane_id();
-			const uint2 r = __ldg(reinterpret_cast<const uint2 *>(cells + base + uint64_t(ia) * W + q));
+			const uint2 r = __ldg(rows + (base + uint64_t(ia) * W + q) * STEP);
 			const uint64_t pos = uint64_t(r.y) + __popc(r.x & below);
 			if (pos < T)
 			{
@@ -428,8 +432,8 @@ void free_mats(Ctx &c, BitMats &mats)
 
 // Lists the triangles of the resident graph into c.dtris (3*T u32) and sets
 // c.T. With keep, the bit matrices stay behind in *keep when they were built in
-// one chunk and their positions fit the edge records (32-bit word positions,
-// 16-bit row positions); else *keep is left empty.
+// one chunk, their positions fit the edge records (32-bit word positions,
+// 16-bit row positions) and there is room for them; else *keep is left empty.
 int list_triangles(Ctx &c, BitMats *keep)
 {
 	c.T = 0;
@@ -438,6 +442,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 	const uint64_t n = c.n, m = c.m;
 	uint64_t *words = nullptr, *woff = nullptr, *aoff = nullptr;
 	uint32_t *rowcnt = nullptr, *cols = nullptr, *err = nullptr;
+	uint2 *rows = nullptr;
 	uint4 *cells = nullptr, *erec = nullptr;
 	int rc = NUCLEUS34_OK;
 	auto cleanup = [&] {
@@ -446,6 +451,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 		c.release(aoff);
 		c.release(rowcnt);
 		c.release(cols);
+		c.release(rows);
 		c.release(cells);
 		c.release(erec);
 		c.release(err);
@@ -475,10 +481,10 @@ int list_triangles(Ctx &c, BitMats *keep)
 		words = nullptr;
 		if ((rc = dalloc(c, &rowcnt, m, "triangles per edge")) || (rc = dalloc(c, &aoff, m + 1, "triangle offsets")))
 			break;
-		// Chunks of sources whose words (a column word and a cell) fit a
-		// quarter of the room left; one chunk when all of them do.
+		// Chunks of sources whose words (a column word, a row word and its
+		// prefix) fit a quarter of the room left; one chunk when all of them do.
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
-		uint64_t cap_words = std::max<uint64_t>(room / 4 / 20, uint64_t(1) << 20);
+		uint64_t cap_words = std::max<uint64_t>(room / 4 / 12, uint64_t(1) << 20);
 		// NUCLEUS34_LIST_CHUNK_WORDS=N caps the chunk at N words (a test hook
 		// for the chunked path, which budgets alone reach only on large graphs)
 		if (const char *e = std::getenv("NUCLEUS34_LIST_CHUNK_WORDS"))
@@ -536,7 +542,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 			maxw = std::max(maxw, hwc[i + 1] - hwc[i]);
 		const uint64_t alloc_w = maxw ? maxw : 1;
 		if ((rc = dalloc(c, &cols, alloc_w, "listing column words")) ||
-			(rc = dalloc(c, &cells, alloc_w, "listing cells")))
+			(rc = dalloc(c, &rows, alloc_w, "listing row words")))
 			break;
 		const size_t nchunks = cuts.size() - 1;
 		auto bits_of_chunk = [&](size_t i) -> int {
@@ -545,7 +551,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 				N34_LAUNCH(c, k_list_cols, grid_for(c, j1 - j0, TRI_WARPS, 32), TRI_THREADS, 0, c.dO, c.dE, c.dsrc,
 						   j0, j1, woff, hwc[i], cols);
 			N34_LAUNCH(c, k_list_rows, grid_for(c, u1 - u0, TRI_WARPS, 32), TRI_THREADS, 0, c.dO, u0, u1, woff,
-					   hwc[i], cols, cells, rowcnt);
+					   hwc[i], cols, rows, rowcnt);
 			return NUCLEUS34_OK;
 		};
 		// counts of every chunk, then the offsets
@@ -576,9 +582,11 @@ int list_triangles(Ctx &c, BitMats *keep)
 		if ((rc = dalloc(c, &c.dtris, 3 * T, "triangles")))
 			break;
 		bool kept = keep && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu;
-		if (kept && dalloc(c, &erec, m, "edge records"))
+		if (kept && (dalloc(c, &erec, m, "edge records") || dalloc(c, &cells, alloc_w, "listing cells")))
 		{
-			erec = nullptr; // the matrices are not kept then
+			c.release(erec);
+			erec = nullptr;
+			cells = nullptr;
 			kept = false;
 			clear_error();
 		}
@@ -591,9 +599,15 @@ int list_triangles(Ctx &c, BitMats *keep)
 			if (j1 > j0)
 			{
 				k_list_ids<<<grid_for(c, j1 - j0, TRI_THREADS, 32), TRI_THREADS, 0, c.stream>>>(
-					c.dO, c.dsrc, j0, j1, woff, hwc[i], aoff, cells, cols, erec);
-				k_list_write<<<grid_for(c, j1 - j0, TRI_WARPS, 32), TRI_THREADS, 0, c.stream>>>(
-					c.dO, c.dE, c.dsrc, j0, j1, woff, hwc[i], cells, T, c.dtris, err);
+					c.dO, c.dsrc, j0, j1, woff, hwc[i], aoff, rows, cols, cells, erec);
+				const uint32_t grid = grid_for(c, j1 - j0, TRI_WARPS, 32);
+				if (kept)
+					k_list_write<2><<<grid, TRI_THREADS, 0, c.stream>>>(c.dO, c.dE, c.dsrc, j0, j1, woff, hwc[i],
+																		 reinterpret_cast<const uint2 *>(cells), T,
+																		 c.dtris, err);
+				else
+					k_list_write<1><<<grid, TRI_THREADS, 0, c.stream>>>(c.dO, c.dE, c.dsrc, j0, j1, woff, hwc[i],
+																		 rows, T, c.dtris, err);
 				c.launches += 2;
 			}
 		}
