@@ -298,16 +298,13 @@ void select_tune(Ctx &c, int variant)
 		c.tune = tune_filled(r->tune);
 }
 
-int run(Ctx &c, int variant, nucleus34_result *out)
+// One pass over the phases. rows: the bit form is allowed; *lists is set when
+// the pass failed for want of memory with the matrices in use, so that the
+// incidence lists alone may still succeed.
+static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_result *out)
 {
-	if (variant != NUCLEUS34_DIRECT && variant != NUCLEUS34_ONDEMAND)
-		return fail(NUCLEUS34_E_INVALID, "unknown variant");
-	if (!c.dO)
-		return fail(NUCLEUS34_E_STATE, "no graph uploaded");
-	N34_TRY(set_device(c));
 	c.release_results();
 	const uint64_t launches0 = c.launches;
-	c.peak = c.in_use;
 	Events ev;
 	if (!ev.ok)
 		return fail(NUCLEUS34_E_CUDA, "event creation");
@@ -326,8 +323,9 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	{
 		c.peel_debit_sec = 0;
 		N34_CUDA(cudaEventRecord(ev.e[0], c.stream));
-		if ((rc = list_triangles(c, bit_form_wanted(c, variant) ? &mats : nullptr)))
+		if ((rc = list_triangles(c, rows ? &mats : nullptr)))
 			break;
+		*lists = mats.cells != nullptr;
 		if ((rc = segments_after_listing(c)))
 			break;
 		N34_CUDA(cudaEventRecord(ev.e[1], c.stream));
@@ -350,6 +348,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 			break;
 		if (!bits)
 			free_mats(c, mats);
+		*lists = bits;
 		if (bits)
 			r.sum_te_sq = in.sum_te_sq;
 		else if (c.T)
@@ -395,26 +394,6 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 		if (variant == NUCLEUS34_DIRECT && total)
 		{
 			rc = bits ? list_cliques_bits(c, mats, in, S, own, csr) : list_cliques(c, inc, S, own, csr);
-			if (bits && rc == NUCLEUS34_E_OOM_BUDGET)
-			{
-				// the incidence lists may be smaller than the rows
-				clear_error();
-				bits = false;
-				free_mats(c, mats);
-				free_in_rows(c, in);
-				free_clique_csr(c, csr);
-				c.release(c.dquds);
-				c.dquds = nullptr;
-				c.release(own);
-				c.release(S);
-				own = nullptr;
-				S = nullptr;
-				if ((rc = build_incidence(c, inc, false, false)) || (rc = dalloc(c, &S, c.T, "support")) ||
-					(rc = dalloc(c, &own, c.T, "clique owner counts")) ||
-					(rc = count_support(c, inc, S, &total, own)))
-					break;
-				rc = list_cliques(c, inc, S, own, csr);
-			}
 			if (rc)
 				break;
 			if (c.Q != total / 4)
@@ -473,6 +452,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	free_in_rows(c, in);
 	c.release(S);
 	c.release(own);
+	*lists = *lists && rc == NUCLEUS34_E_OOM_BUDGET;
 	if (rc)
 	{
 		c.release_results();
@@ -501,6 +481,25 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	if (out)
 		*out = r;
 	return NUCLEUS34_OK;
+}
+
+int run(Ctx &c, int variant, nucleus34_result *out)
+{
+	if (variant != NUCLEUS34_DIRECT && variant != NUCLEUS34_ONDEMAND)
+		return fail(NUCLEUS34_E_INVALID, "unknown variant");
+	if (!c.dO)
+		return fail(NUCLEUS34_E_STATE, "no graph uploaded");
+	N34_TRY(set_device(c));
+	c.peak = c.in_use;
+	bool lists = false;
+	int rc = run_phases(c, variant, bit_form_wanted(c, variant), &lists, out);
+	if (rc && lists)
+	{
+		// the incidence lists may be smaller than the rows
+		clear_error();
+		rc = run_phases(c, variant, false, &lists, out);
+	}
+	return rc;
 }
 
 // Pinned buffers for large results on their way to pageable host memory,

@@ -565,9 +565,10 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 			break;
 		}
 		// the in-rows and their triangles, the counts; then support, k, two
-		// frontiers and the ordering bitmap
+		// frontiers, the ordering bitmap and, if kept, the death rounds
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
-		if (in.nwords > 0xffffffffull || 16 * in.nwords + 20 * T + T / 8 + 16 * m + (uint64_t(1) << 20) > room)
+		const uint64_t per_tri = c.opt_flags & NUCLEUS34_OPT_VERIFIABLE ? 24 : 20;
+		if (in.nwords > 0xffffffffull || 16 * in.nwords + per_tri * T + T / 8 + 16 * m + (uint64_t(1) << 20) > room)
 			break;
 		if ((rc = dalloc(c, &in.cells, in.nwords, "in-rows")) || (rc = dalloc(c, &in.live, m, "in-row counts")) ||
 			(rc = dalloc(c, &cnt, m, "in-row counts")) || (rc = dalloc(c, &sumsq, 1, "square sum")))

@@ -51,3 +51,22 @@ def test_listing_room(n34, oracle, make, variant):
     d = n34.decompose(g, variant=variant, mem_budget_bytes=budget, n_quds=0)
     assert np.array_equal(d.k, o.k) and np.array_equal(d.tris, o.tris)
     assert d.result["peak_device_bytes"] <= budget
+
+
+def test_death_rounds_room(n34, oracle):
+    """Budgets from the memory-lean lists' need to that of the rows with every
+    table, with the death rounds kept: a graph of 10 triangles and 12 words an
+    edge, where the rows need more without death rounds than the lists with
+    them."""
+    g = n34.graph_from_edges(*dense(3000, 0.1, 2))
+    o = oracle.decompose(g, quds_cap=0)
+    full, low = (n34.decompose(g, variant="ondemand", flags=n34.OPT_VERIFIABLE | fl, n_quds=0)
+                 .result["peak_device_bytes"] for fl in (0, n34.OPT_LEAN_MEMORY))
+    assert low < full
+    for i in range(33):
+        budget = low + (full - low) * i // 32 + (1 << 20)
+        with n34.Context(mem_budget_bytes=budget, flags=n34.OPT_VERIFIABLE) as ctx:
+            ctx.upload(g)
+            r = ctx.run("ondemand")
+            assert r["peak_device_bytes"] <= budget
+            assert np.array_equal(ctx.copy_k(r["triangle_count"]), o.k)
