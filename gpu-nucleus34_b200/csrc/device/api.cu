@@ -299,8 +299,9 @@ void select_tune(Ctx &c, int variant)
 }
 
 // One pass over the phases. rows: the bit form is allowed; *lists is set when
-// the pass failed for want of memory with the matrices in use, so that the
-// incidence lists alone may still succeed.
+// the pass failed with the matrices in use, for want of memory or because the
+// rows do not suit the graph's orientation, so that the incidence lists alone may
+// still succeed.
 static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_result *out)
 {
 	c.release_results();
@@ -318,7 +319,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	uint32_t *own = nullptr;
 	int rc = NUCLEUS34_OK;
 	PeelCtl pc{};
-	bool peeled = false;
+	bool peeled = false, acyclic = true;
 	do
 	{
 		c.peel_debit_sec = 0;
@@ -379,8 +380,14 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 				break;
 			if (variant == NUCLEUS34_DIRECT && (rc = dalloc(c, &own, c.T, "clique owner counts")))
 				break;
-			if ((rc = bits ? count_support_bits(c, mats, in, S, &total, own) : count_support(c, inc, S, &total, own)))
+			if ((rc = bits ? count_support_bits(c, mats, in, S, &total, own, &acyclic)
+						   : count_support(c, inc, S, &total, own)))
 				break;
+			if (!acyclic)
+			{
+				rc = fail(NUCLEUS34_E_INVALID, "the orientation has a directed cycle");
+				break;
+			}
 			if (total % 4)
 			{
 				rc = fail(NUCLEUS34_E_CUDA, "internal: clique incidences not a multiple of 4");
@@ -452,7 +459,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	free_in_rows(c, in);
 	c.release(S);
 	c.release(own);
-	*lists = *lists && rc == NUCLEUS34_E_OOM_BUDGET;
+	*lists = *lists && (rc == NUCLEUS34_E_OOM_BUDGET || !acyclic);
 	if (rc)
 	{
 		c.release_results();
@@ -495,7 +502,7 @@ int run(Ctx &c, int variant, nucleus34_result *out)
 	int rc = run_phases(c, variant, bit_form_wanted(c, variant), &lists, out);
 	if (rc && lists)
 	{
-		// the incidence lists may be smaller than the rows
+		// the incidence lists may be smaller than the rows, and suit any orientation
 		clear_error();
 		rc = run_phases(c, variant, false, &lists, out);
 	}

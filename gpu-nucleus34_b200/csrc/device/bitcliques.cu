@@ -96,7 +96,10 @@ __global__ void k_above(const uint32_t *__restrict__ O, const uint32_t *__restri
 
 // support[t] = cliques on t: the common bits of its two rows and of its two
 // in-rows, one thread per triangle (neighbours share their source, so the rows
-// come from L1). With OWN also the cliques whose lowest triangle is t.
+// come from L1). With OWN also the cliques whose lowest triangle is t. total:
+// cliques found in the rows and in the in-rows, over all triangles. A clique is
+// in the rows of three of its triangles and in the in-rows of the fourth; three
+// vertices above a source that form a directed cycle are in the rows alone.
 template <bool OWN>
 __global__ void __launch_bounds__(CL_THREADS) k_support_bits(
 	const uint32_t *__restrict__ tris, uint64_t T, const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_support_bits(
 	const uint2 *__restrict__ above, int32_t *__restrict__ support, uint32_t *__restrict__ own,
 	unsigned long long *__restrict__ total)
 {
-	unsigned long long acc = 0;
+	unsigned long long acc[2] = {0, 0};
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < T; t += stride)
 	{
@@ -122,6 +125,8 @@ __global__ void __launch_bounds__(CL_THREADS) k_support_bits(
 			else
 				cnt += __popc(__ldg(&rows[r.ra.x + q].z) & __ldg(&rows[r.rb.x + q].z));
 		}
+		acc[0] += cnt;
+		acc[1] -= cnt;
 		if (la.x && lb.x)
 			for (uint32_t q = 0; q < la.y; ++q)
 			{
@@ -133,13 +138,17 @@ __global__ void __launch_bounds__(CL_THREADS) k_support_bits(
 		support[t] = int32_t(cnt);
 		if (OWN)
 			own[t] = mine;
-		acc += cnt;
+		acc[1] += cnt;
 	}
 #pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		acc += __shfl_xor_sync(FULL, acc, o);
-	if (lane_id() == 0 && acc)
-		atomicAdd(total, acc);
+	for (int i = 0; i < 2; ++i)
+	{
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1)
+			acc[i] += __shfl_xor_sync(FULL, acc[i], o);
+		if (lane_id() == 0 && acc[i])
+			atomicAdd(total + i, acc[i]);
+	}
 }
 
 __device__ __forceinline__ void sort2(uint32_t &a, uint32_t &b)
@@ -308,14 +317,14 @@ static int build_above(Ctx &c, const InMats &in, uint2 **above)
 }
 
 int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total,
-					   uint32_t *own)
+					   uint32_t *own, bool *acyclic)
 {
-	unsigned long long *dtot = nullptr, h = 0;
+	unsigned long long *dtot = nullptr, h[2] = {0, 0};
 	uint2 *above = nullptr;
-	int rc = dalloc(c, &dtot, 1, "support total");
+	int rc = dalloc(c, &dtot, 2, "support total");
 	if (!rc && own)
 		rc = build_above(c, in, &above);
-	if (!rc && cudaMemsetAsync(dtot, 0, 8, c.stream) != cudaSuccess)
+	if (!rc && cudaMemsetAsync(dtot, 0, 16, c.stream) != cudaSuccess)
 		rc = fail(NUCLEUS34_E_CUDA, "memset");
 	if (!rc)
 	{
@@ -328,13 +337,14 @@ int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *s
 																	 in.live, c.dsrc, above, support, own, dtot);
 		c.launches++;
 		if (cudaGetLastError() != cudaSuccess ||
-			cudaMemcpyAsync(&h, dtot, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaMemcpyAsync(h, dtot, 16, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
 			cudaStreamSynchronize(c.stream) != cudaSuccess)
 			rc = fail(NUCLEUS34_E_CUDA, "support count");
 	}
 	c.release(dtot);
 	c.release(above);
-	*total = h;
+	*total = h[0] + h[1];
+	*acyclic = h[0] == 3 * h[1];
 	return rc;
 }
 

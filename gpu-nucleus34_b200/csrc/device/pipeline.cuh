@@ -101,13 +101,16 @@ int segments_after_peel(Ctx &c);
 // The bit-matrix form of the support count, the clique list and the peel.
 bool bit_form_wanted(const Ctx &c, int variant);
 // Builds the in-rows; *fits is false, and nothing is left, when they and what
-// the form needs beside them exceed the room left. by_source: columns ascend
+// the form needs beside them exceed the room left, or when the graph has an edge
+// in both directions. by_source: columns ascend
 // with the in-edge's source.
 int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits);
 void free_in_rows(Ctx &c, InMats &in);
-// own (optional, needs by_source): cliques whose lowest triangle is t.
+// own (optional, needs by_source): cliques whose lowest triangle is t. *acyclic:
+// no three vertices above one source form a directed cycle (the rows would take
+// them for a clique).
 int count_support_bits(Ctx &c, const BitMats &mats, const InMats &in, int32_t *support, uint64_t *total,
-					   uint32_t *own);
+					   uint32_t *own, bool *acyclic);
 // Direct variant: the clique list and, where the peel uses them in place of the
 // rows (which it then gives back), the triangle -> clique lists.
 int list_cliques_bits(Ctx &c, BitMats &mats, InMats &in, const int32_t *support, const uint32_t *own,
