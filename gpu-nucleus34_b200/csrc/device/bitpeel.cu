@@ -76,21 +76,13 @@ __global__ void k_in_sorted_columns(const uint32_t *__restrict__ E, const unsign
 	}
 }
 
-// cells of every edge's in-row; *both: there are edges u -> v and v -> u, whose
-// triangles the rows do not tell apart
-__global__ void k_in_widths(const uint32_t *__restrict__ O, const uint32_t *__restrict__ E,
-							const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
-							uint32_t *__restrict__ width, uint32_t *__restrict__ both)
+// cells of every edge's in-row
+__global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
+							uint32_t *__restrict__ width)
 {
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
-	{
-		const uint32_t u = src[e], v = __ldg(E + e), end = __ldg(O + v + 1);
-		width[e] = (indeg[u] + 31) >> 5;
-		const uint32_t at = lower_bound32(E, __ldg(O + v), end, u);
-		if (at < end && __ldg(E + at) == u)
-			*both = 1;
-	}
+		width[e] = (indeg[src[e]] + 31) >> 5;
 }
 
 __global__ void k_in_starts(const uint64_t *__restrict__ off, uint64_t m, uint4 *__restrict__ erec)
@@ -519,21 +511,23 @@ struct BitPath
 } // namespace
 
 // The bit form serves the direct variant, and the on-demand variant unless a
-// flag asks for the list form (a layout, an owner test or a schedule of it).
+// flag asks for the list form (a layout, an owner test or a schedule of it); a
+// graph with an edge in both directions goes to the lists, as one bit would stand
+// for two triangles.
 bool bit_form_wanted(const Ctx &c, int variant)
 {
 	constexpr uint32_t LIST_FORM = NUCLEUS34_OPT_STAMP_PEEL | NUCLEUS34_OPT_LEAN_MEMORY | NUCLEUS34_OPT_HOST_LOOP |
 								   NUCLEUS34_OPT_NO_SMALL_ROUNDS | NUCLEUS34_OPT_FRONTIER_BY_C |
 								   NUCLEUS34_OPT_CHUNKED_DEBIT | NUCLEUS34_OPT_SCALAR_SCANS |
 								   NUCLEUS34_OPT_PIPELINED_DEBIT | NUCLEUS34_OPT_DEBIT_CURSOR;
-	return variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM);
+	return c.one_way && (variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM));
 }
 
 int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits)
 {
 	const uint64_t T = c.T, m = c.m;
 	*fits = false;
-	uint32_t *indeg = nullptr, *width = nullptr, *cnt = nullptr, *both = nullptr, hboth = 0;
+	uint32_t *indeg = nullptr, *width = nullptr, *cnt = nullptr;
 	uint64_t *off = nullptr;
 	unsigned long long *sumsq = nullptr;
 	const uint32_t gm = grid_for(c, m, 256), gt = grid_for(c, T, 256);
@@ -541,16 +535,15 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 	do
 	{
 		if ((rc = dalloc(c, &indeg, c.n, "in-degrees")) || (rc = dalloc(c, &width, m, "in-row widths")) ||
-			(rc = dalloc(c, &off, m + 1, "in-row offsets")) || (rc = dalloc(c, &both, 1, "orientation check")))
+			(rc = dalloc(c, &off, m + 1, "in-row offsets")))
 			break;
-		if (cudaMemsetAsync(indeg, 0, c.n * 4, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(both, 0, 4, c.stream) != cudaSuccess)
+		if (cudaMemsetAsync(indeg, 0, c.n * 4, c.stream) != cudaSuccess)
 		{
 			rc = fail(NUCLEUS34_E_CUDA, "memset");
 			break;
 		}
 		k_in_columns<<<gm, 256, 0, c.stream>>>(c.dE, m, indeg, mats.erec);
-		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dO, c.dE, c.dsrc, m, indeg, width, both);
+		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dsrc, m, indeg, width);
 		c.launches += 2;
 		if (by_source)
 		{
@@ -568,14 +561,11 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 		if ((rc = scan_u32(c, width, off, m)))
 			break;
 		if (cudaMemcpyAsync(&in.nwords, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaMemcpyAsync(&hboth, both, 4, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
 			cudaStreamSynchronize(c.stream) != cudaSuccess)
 		{
 			rc = fail(NUCLEUS34_E_CUDA, "in-row widths");
 			break;
 		}
-		if (hboth)
-			break;
 		// the in-rows and their triangles, the counts; then support, k, two
 		// frontiers, the ordering bitmap and, if kept, the death rounds
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
@@ -617,7 +607,6 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 	c.release(indeg);
 	c.release(width);
 	c.release(cnt);
-	c.release(both);
 	c.release(off);
 	c.release(sumsq);
 	if (rc || !*fits)

@@ -111,6 +111,7 @@ struct Ctx
 	// resident graph
 	uint64_t n = 0, m = 0;
 	uint32_t max_out = 0;   // maximum out-degree (the tune table's skew class)
+	bool one_way = true;    // no edge is there in both directions
 	uint32_t *dO = nullptr; // n+1
 	uint32_t *dE = nullptr; // m
 	uint32_t *dsrc = nullptr; // m

@@ -101,9 +101,8 @@ int segments_after_peel(Ctx &c);
 // The bit-matrix form of the support count, the clique list and the peel.
 bool bit_form_wanted(const Ctx &c, int variant);
 // Builds the in-rows; *fits is false, and nothing is left, when they and what
-// the form needs beside them exceed the room left, or when the graph has an edge
-// in both directions. by_source: columns ascend
-// with the in-edge's source.
+// the form needs beside them exceed the room left. by_source: columns ascend with
+// the in-edge's source.
 int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits);
 void free_in_rows(Ctx &c, InMats &in);
 // own (optional, needs by_source): cliques whose lowest triangle is t. *acyclic:
