@@ -335,7 +335,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	{
 		c.peel_debit_sec = 0;
 		N34_CUDA(cudaEventRecord(ev.e[0], c.stream));
-		if ((rc = list_triangles(c, rows ? &mats : nullptr)))
+		if ((rc = list_triangles(c, rows ? &mats : nullptr, rows_least_triangles(c, variant))))
 			break;
 		*lists = mats.cells != nullptr;
 		if ((rc = segments_after_listing(c)))
@@ -353,10 +353,11 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 			break;
 		}
 		c.lean_run = false;
-		// both variants run on the listing's bit matrices when they were kept and
-		// the rest fits beside them, else on the incidence lists
+		// both variants run on the listing's bit matrices when they were kept, the
+		// rest fits beside them and they are the less work, else on the incidence
+		// lists
 		bool bits = c.T && mats.cells;
-		if (bits && (rc = build_in_rows(c, mats, in, variant == NUCLEUS34_DIRECT, &bits)))
+		if (bits && (rc = build_in_rows(c, mats, in, variant, &bits)))
 			break;
 		if (!bits)
 			free_mats(c, mats);

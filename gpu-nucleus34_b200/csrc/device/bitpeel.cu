@@ -37,6 +37,8 @@
 // four batches in flight changed nothing: latency is not the bound.
 #include "pipeline.cuh"
 
+#include <algorithm>
+
 #include "peel_loop.cuh"
 
 namespace n34 {
@@ -76,13 +78,60 @@ __global__ void k_in_sorted_columns(const uint32_t *__restrict__ E, const unsign
 	}
 }
 
-// cells of every edge's in-row
-__global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
-							uint32_t *__restrict__ width)
+// What the rows and the lists would cost (rows_pay), summed over the edges.
+struct EdgeSums
 {
+	unsigned long long sum_sq;  // of the triangles on an edge (k_in_counts)
+	unsigned long long words;   // row and in-row words of all triangles
+	unsigned long long heads;   // sum over triangles of the triangles whose head or tail edge is
+	unsigned long long tails;   // theirs: of their head edge, of their tail edge
+};
+
+// v of all threads of the block to *sum (all threads call)
+__device__ __forceinline__ void block_sum(unsigned long long v, unsigned long long *sum)
+{
+	__shared__ unsigned long long s_sum;
+	if (threadIdx.x == 0)
+		s_sum = 0;
+	__syncthreads();
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		v += __shfl_xor_sync(FULL, v, o);
+	if (lane_id() == 0 && v)
+		atomicAdd(&s_sum, v);
+	__syncthreads();
+	if (threadIdx.x == 0 && s_sum)
+		atomicAdd(sum, s_sum);
+	__syncthreads();
+}
+
+// cells of every edge's in-row; cnt: triangles whose head or tail edge it is
+__global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
+							const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
+							uint32_t *__restrict__ width, uint32_t *__restrict__ cnt, EdgeSums *__restrict__ sums)
+{
+	unsigned long long words = 0, heads = 0, tails = 0;
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
-		width[e] = (indeg[src[e]] + 31) >> 5;
+	{
+		const uint2 r = __ldg(reinterpret_cast<const uint2 *>(erec + e));
+		const uint32_t W = r.y >> 16, in = (indeg[src[e]] + 31) >> 5;
+		uint32_t head = 0, sym = 0;
+		for (uint32_t q = 0; q < W; ++q)
+		{
+			const uint4 c = __ldg(rows + r.x + q);
+			head += __popc(c.x);
+			sym += __popc(c.z);
+		}
+		width[e] = in;
+		cnt[e] = sym;
+		words += uint64_t(head) * (W + in);
+		heads += uint64_t(head) * sym;
+		tails += uint64_t(sym - head) * sym;
+	}
+	block_sum(words, &sums->words);
+	block_sum(heads, &sums->heads);
+	block_sum(tails, &sums->tails);
 }
 
 __global__ void k_in_starts(const uint64_t *__restrict__ off, uint64_t m, uint4 *__restrict__ erec)
@@ -104,34 +153,26 @@ __global__ void k_in_set(const uint32_t *__restrict__ tris, uint64_t T, const ui
 	}
 }
 
-// triangles per in-row, and the sum over edges of (triangles on the edge)^2:
-// those with the edge as a or b are in its symmetric row
-__global__ void k_in_counts(const uint4 *__restrict__ erec, uint64_t m, const uint4 *__restrict__ rows,
-							const uint4 *__restrict__ cells, const uint32_t *__restrict__ width,
-							uint32_t *__restrict__ cnt, uint2 *__restrict__ live,
-							unsigned long long *__restrict__ sum_sq)
+// triangles per in-row, in place of those with the edge as head or tail, and the
+// sum over edges of (triangles on the edge)^2
+__global__ void k_in_counts(const uint4 *__restrict__ erec, uint64_t m, const uint4 *__restrict__ cells,
+							const uint32_t *__restrict__ width, uint32_t *__restrict__ cnt,
+							uint2 *__restrict__ live, unsigned long long *__restrict__ sum_sq)
 {
 	unsigned long long acc = 0;
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
 	{
-		const uint4 r = erec[e];
-		const uint32_t W = width[e];
+		const uint32_t first = erec[e].z, W = width[e], rest = cnt[e];
 		uint32_t n = 0;
 		for (uint32_t q = 0; q < W; ++q)
-			n += __popc(cells[r.z + q].x);
+			n += __popc(cells[first + q].x);
+		const unsigned long long d = uint64_t(n) + rest;
 		cnt[e] = n;
 		live[e] = make_uint2(n, W);
-		unsigned long long d = n;
-		for (uint32_t q = 0; q < (r.y >> 16); ++q)
-			d += __popc(rows[r.x + q].z);
 		acc += d * d;
 	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		acc += __shfl_xor_sync(FULL, acc, o);
-	if (lane_id() == 0 && acc)
-		atomicAdd(sum_sq, acc);
+	block_sum(acc, sum_sq);
 }
 
 // first positions of the cells' triangles in tri; all not dead, none dying. A
@@ -523,28 +564,73 @@ bool bit_form_wanted(const Ctx &c, int variant)
 	return c.one_way && (variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM));
 }
 
-int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits)
+// The rows are worth their words: every triangle's words are read in the support
+// count and once more when it dies, however few bits they hold, where the lists
+// cost by what they hold. `lists` is the lesser of the entries on the triangles'
+// head and tail edges (those with the edge as head or tail: the others are not
+// counted before the in-rows are built). Words and entries of R-MAT and geometric
+// graphs are 0.1 to 1.1 to one. Hubs that are joined to each other and to many
+// vertices of degree 1 to 3 (in-rows long and nearly empty) cross over between
+// 2.9 and 4.7 on demand, where the lists' rounds take longer (incidence, support
+// and peel, rows against lists, ms: 8.1 and 14.1 at 1.1, 14.7 and 15.6 at 2.9,
+// 20.5 and 15.6 at 4.7, 94 and 33 at 26), and between 1.5 and 2 in the direct
+// variant, which peels over the clique list in either form (19.7 and 25 at 1.5,
+// 19.0 and 15.5 at 2.0, 237 and 32 at 26). On demand the lists also take 1 to 2
+// ms for the launches of their rounds: the time of 1e8 words.
+static bool rows_pay(int variant, uint64_t words, uint64_t lists)
+{
+	return variant == NUCLEUS34_DIRECT ? words <= lists + lists / 2 : words <= 3 * lists + lists / 2 + 100000000;
+}
+
+// From this many triangles on the listing keeps its matrices: building in-rows is
+// several passes over the edges, whatever the triangles. On demand that is 0.03
+// ns an edge against 1 ms for the launches of the lists' rounds (if any: road-like
+// grids have no cliques); the direct variant also sorts the in-edges, 0.2 ns an
+// edge, and has no such launches. Incidence, support, cliques and peel, rows against
+// lists, ms: on demand, 2e6 edges and 2e5 triangles 0.25 and 0.26, 3.2e7 and 6e5
+// 1.86 and 0.98, 1.2e7 and 4e4 (with rounds) 1.2 and 1.5; direct, 8e6 and 1.5e6
+// 2.0 and 1.3, 6e6 and 3.5e6 2.76 and 2.81, 1e7 and 1e7 5.7 and 7.4.
+uint64_t rows_least_triangles(const Ctx &c, int variant)
+{
+	return variant == NUCLEUS34_DIRECT ? c.m / 2 : c.m > (uint64_t(1) << 23) ? c.m / 16 : 0;
+}
+
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fits)
 {
 	const uint64_t T = c.T, m = c.m;
+	const bool by_source = variant == NUCLEUS34_DIRECT;
 	*fits = false;
 	uint32_t *indeg = nullptr, *width = nullptr, *cnt = nullptr;
 	uint64_t *off = nullptr;
-	unsigned long long *sumsq = nullptr;
+	EdgeSums *sums = nullptr, hsums{};
 	const uint32_t gm = grid_for(c, m, 256), gt = grid_for(c, T, 256);
 	int rc = NUCLEUS34_OK;
 	do
 	{
 		if ((rc = dalloc(c, &indeg, c.n, "in-degrees")) || (rc = dalloc(c, &width, m, "in-row widths")) ||
+			(rc = dalloc(c, &cnt, m, "in-row counts")) || (rc = dalloc(c, &sums, 1, "edge sums")) ||
 			(rc = dalloc(c, &off, m + 1, "in-row offsets")))
 			break;
-		if (cudaMemsetAsync(indeg, 0, c.n * 4, c.stream) != cudaSuccess)
+		if (cudaMemsetAsync(indeg, 0, c.n * 4, c.stream) != cudaSuccess ||
+			cudaMemsetAsync(sums, 0, sizeof(EdgeSums), c.stream) != cudaSuccess)
 		{
 			rc = fail(NUCLEUS34_E_CUDA, "memset");
 			break;
 		}
 		k_in_columns<<<gm, 256, 0, c.stream>>>(c.dE, m, indeg, mats.erec);
-		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dsrc, m, indeg, width);
+		k_in_widths<<<gm, 256, 0, c.stream>>>(c.dsrc, m, indeg, mats.erec, mats.cells, width, cnt, sums);
 		c.launches += 2;
+		if ((rc = scan_u32(c, width, off, m)))
+			break;
+		if (cudaMemcpyAsync(&in.nwords, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaMemcpyAsync(&hsums, sums, sizeof(EdgeSums), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+			cudaStreamSynchronize(c.stream) != cudaSuccess)
+		{
+			rc = fail(NUCLEUS34_E_CUDA, "in-row widths");
+			break;
+		}
+		if (!rows_pay(variant, hsums.words, std::min(hsums.heads, hsums.tails)))
+			break;
 		if (by_source)
 		{
 			if ((rc = dalloc(c, &in.in_off, c.n + 1, "in-edge offsets")) || (rc = scan_u32(c, indeg, in.in_off, c.n)) ||
@@ -558,32 +644,22 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 		}
 		c.release(indeg);
 		indeg = nullptr;
-		if ((rc = scan_u32(c, width, off, m)))
-			break;
-		if (cudaMemcpyAsync(&in.nwords, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaStreamSynchronize(c.stream) != cudaSuccess)
-		{
-			rc = fail(NUCLEUS34_E_CUDA, "in-row widths");
-			break;
-		}
 		// the in-rows and their triangles, the counts; then support, k, two
 		// frontiers, the ordering bitmap and, if kept, the death rounds
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
 		const uint64_t per_tri = c.opt_flags & NUCLEUS34_OPT_VERIFIABLE ? 24 : 20;
 		if (in.nwords > 0xffffffffull || 16 * in.nwords + per_tri * T + T / 8 + 16 * m + (uint64_t(1) << 20) > room)
 			break;
-		if ((rc = dalloc(c, &in.cells, in.nwords, "in-rows")) || (rc = dalloc(c, &in.live, m, "in-row counts")) ||
-			(rc = dalloc(c, &cnt, m, "in-row counts")) || (rc = dalloc(c, &sumsq, 1, "square sum")))
+		if ((rc = dalloc(c, &in.cells, in.nwords, "in-rows")) || (rc = dalloc(c, &in.live, m, "in-row counts")))
 			break;
-		if (cudaMemsetAsync(in.cells, 0, in.nwords * 16, c.stream) != cudaSuccess ||
-			cudaMemsetAsync(sumsq, 0, 8, c.stream) != cudaSuccess)
+		if (cudaMemsetAsync(in.cells, 0, in.nwords * 16, c.stream) != cudaSuccess)
 		{
 			rc = fail(NUCLEUS34_E_CUDA, "memset");
 			break;
 		}
 		k_in_starts<<<gm, 256, 0, c.stream>>>(off, m, mats.erec);
 		k_in_set<<<gt, 256, 0, c.stream>>>(c.dtris, T, mats.erec, in.cells);
-		k_in_counts<<<gm, 256, 0, c.stream>>>(mats.erec, m, mats.cells, in.cells, width, cnt, in.live, sumsq);
+		k_in_counts<<<gm, 256, 0, c.stream>>>(mats.erec, m, in.cells, width, cnt, in.live, &sums->sum_sq);
 		c.launches += 3;
 		if ((rc = scan_u32(c, cnt, off, m)))
 			break;
@@ -593,7 +669,7 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 		k_in_place<<<gt, 256, 0, c.stream>>>(c.dtris, T, mats.erec, in.cells, in.tri);
 		c.launches += 2;
 		uint64_t placed = 0;
-		if (cudaMemcpyAsync(&in.sum_te_sq, sumsq, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+		if (cudaMemcpyAsync(&in.sum_te_sq, &sums->sum_sq, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
 			cudaMemcpyAsync(&placed, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
 			cudaStreamSynchronize(c.stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
 		{
@@ -608,7 +684,7 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool 
 	c.release(width);
 	c.release(cnt);
 	c.release(off);
-	c.release(sumsq);
+	c.release(sums);
 	if (rc || !*fits)
 		free_in_rows(c, in);
 	if (rc == NUCLEUS34_E_OOM_BUDGET)

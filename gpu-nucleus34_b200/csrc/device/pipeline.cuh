@@ -75,7 +75,7 @@ cudaError_t launch_tri_count(const uint32_t *O, const uint32_t *E, uint64_t n, u
 							 cudaStream_t s);
 cudaError_t launch_tri_write(const uint32_t *O, const uint32_t *E, uint64_t n, const uint64_t *toff,
 							 uint32_t *tris, int sm_count, cudaStream_t s);
-int list_triangles(Ctx &c, BitMats *keep);
+int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min);
 void free_mats(Ctx &c, BitMats &mats);
 // lean: no 64-bit key array (entries sorted in place as pairs) and no tpos.
 int build_incidence(Ctx &c, Incidence &inc, bool want_tpos, bool lean = false);
@@ -101,9 +101,11 @@ int segments_after_peel(Ctx &c);
 // The bit-matrix form of the support count, the clique list and the peel.
 bool bit_form_wanted(const Ctx &c, int variant);
 // Builds the in-rows; *fits is false, and nothing is left, when they and what
-// the form needs beside them exceed the room left. by_source: columns ascend with
-// the in-edge's source.
-int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, bool by_source, bool *fits);
+// the form needs beside them exceed the room left, or when the lists are the less
+// work. In the direct variant columns ascend with the in-edge's source (by_source).
+int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fits);
+// Fewest triangles from which on the form may pay.
+uint64_t rows_least_triangles(const Ctx &c, int variant);
 void free_in_rows(Ctx &c, InMats &in);
 // own (optional, needs by_source): cliques whose lowest triangle is t. *acyclic:
 // no three vertices above one source form a directed cycle (the rows would take

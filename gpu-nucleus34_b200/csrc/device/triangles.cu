@@ -431,10 +431,11 @@ void free_mats(Ctx &c, BitMats &mats)
 }
 
 // Lists the triangles of the resident graph into c.dtris (3*T u32) and sets
-// c.T. With keep, the bit matrices stay behind in *keep when they were built in
-// one chunk, their positions fit the edge records (32-bit word positions,
-// 16-bit row positions) and there is room for them; else *keep is left empty.
-int list_triangles(Ctx &c, BitMats *keep)
+// c.T. With keep, the bit matrices stay behind in *keep when there are at least
+// keep_min triangles, they were built in one chunk, their positions fit the edge
+// records (32-bit word positions, 16-bit row positions) and there is room for
+// them; else *keep is left empty.
+int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min)
 {
 	c.T = 0;
 	if (c.m == 0)
@@ -581,7 +582,7 @@ int list_triangles(Ctx &c, BitMats *keep)
 		}
 		if ((rc = dalloc(c, &c.dtris, 3 * T, "triangles")))
 			break;
-		bool kept = keep && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu;
+		bool kept = keep && T >= keep_min && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu;
 		if (kept && (dalloc(c, &erec, m, "edge records") || dalloc(c, &cells, alloc_w, "listing cells")))
 		{
 			c.release(erec);
