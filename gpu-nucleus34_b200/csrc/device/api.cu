@@ -309,6 +309,17 @@ void select_tune(Ctx &c, int variant)
 		c.tune = tune_filled(r->tune);
 }
 
+// Limits the context's budget to what the bit form may use, until lift().
+struct RowsBudget
+{
+	Ctx &c;
+	const uint64_t full;
+	explicit RowsBudget(Ctx &ctx) : c(ctx), full(ctx.budget) {}
+	~RowsBudget() { lift(); }
+	void limit() { c.budget = std::min(full, c.rows_budget); }
+	void lift() { c.budget = full; }
+};
+
 // One pass over the phases. rows: the bit form is allowed; *lists is set when
 // the pass failed with the matrices in use, for want of memory or because the
 // rows do not suit the graph's orientation, so that the incidence lists alone may
@@ -317,6 +328,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 {
 	c.release_results();
 	const uint64_t launches0 = c.launches;
+	RowsBudget budget(c);
 	Events ev;
 	if (!ev.ok)
 		return fail(NUCLEUS34_E_CUDA, "event creation");
@@ -338,6 +350,8 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 		if ((rc = list_triangles(c, rows ? &mats : nullptr, rows_least_triangles(c, variant))))
 			break;
 		*lists = mats.cells != nullptr;
+		if (mats.cells)
+			budget.limit();
 		if ((rc = segments_after_listing(c)))
 			break;
 		N34_CUDA(cudaEventRecord(ev.e[1], c.stream));
@@ -360,7 +374,10 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 		if (bits && (rc = build_in_rows(c, mats, in, variant, &bits)))
 			break;
 		if (!bits)
+		{
 			free_mats(c, mats);
+			budget.lift();
+		}
 		*lists = bits;
 		if (bits)
 			r.sum_te_sq = in.sum_te_sq;

@@ -96,6 +96,9 @@ struct Ctx
 	int sm_count = 148;
 	cudaStream_t stream = nullptr;
 	uint64_t budget = 0;
+	// the part of it that the bit form may use: what a serving pass was admitted
+	// with, while the other passes of its slot use the rest
+	uint64_t rows_budget = ~uint64_t(0);
 	uint64_t in_use = 0;
 	uint64_t peak = 0;
 	uint64_t launches = 0;

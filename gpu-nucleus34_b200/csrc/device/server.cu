@@ -78,6 +78,10 @@ struct Request
 // The admission constants (bytes per triangle, edge and clique bound) and
 // the default direct share live with the estimates in admission.h.
 
+// Added to a pass's admission, as far as the slot has it: the fixed part of what
+// the bit form wants (build_in_rows), which the estimates of small graphs lack.
+constexpr uint64_t PASS_SLACK = 4ull << 20;
+
 struct Slot
 {
 	int device = 0;
@@ -272,12 +276,17 @@ void worker_loop(nucleus34_server_s *s, size_t wi)
 				batch.push_back(q);
 				s->pending.erase(s->pending.begin() + std::ptrdiff_t(i));
 			}
+			take_bytes += std::min(PASS_SLACK, free_b > take_bytes ? free_b - take_bytes : 0);
 			slot.in_flight += take_bytes;
 			s->busy_workers++;
 			const auto now = clk::now();
 			for (auto &q : batch)
 				q->t_start = now;
 		}
+		// rows and in-rows grow with the edges and in-degrees, lists with the
+		// triangles, which the estimates count: a pass keeps to the lists where
+		// the rows would take more than it was admitted with
+		c.rows_budget = take_bytes;
 		serve_union(s, slot, c, batch, direct);
 		{
 			std::lock_guard<std::mutex> lk(s->mu);

@@ -582,7 +582,8 @@ int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min)
 		}
 		if ((rc = dalloc(c, &c.dtris, 3 * T, "triangles")))
 			break;
-		bool kept = keep && T >= keep_min && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu;
+		bool kept = keep && T >= keep_min && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu &&
+					c.in_use + 16 * (m + alloc_w) + 512 <= c.rows_budget;
 		if (kept && (dalloc(c, &erec, m, "edge records") || dalloc(c, &cells, alloc_w, "listing cells")))
 		{
 			c.release(erec);

@@ -15,7 +15,10 @@ namespace n34 {
 // direct variant adds its clique list and triangle->clique incidence (16 +
 // 16 bytes per clique) and one destroyed flag per clique. Applied to the
 // out-wedge and out-triple bounds, not to the true counts, so they
-// overestimate; the GPU tests check them against measured peaks.
+// overestimate where wedges outnumber edges; the GPU tests check them against
+// measured peaks. The rows of the bit form grow with in-degrees too, which
+// they do not know: a pass whose rows would take more than it was admitted
+// with runs on the incidence lists.
 constexpr uint64_t PASS_BYTES_PER_TRIANGLE = 80;
 constexpr uint64_t PASS_BYTES_PER_EDGE = 40;
 constexpr uint64_t DIRECT_BYTES_PER_CLIQUE = 33;
