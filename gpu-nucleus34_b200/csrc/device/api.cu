@@ -378,7 +378,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 			free_mats(c, mats);
 			budget.lift();
 		}
-		*lists = bits;
+		*lists = c.rows_run = bits;
 		if (bits)
 			r.sum_te_sq = in.sum_te_sq;
 		else if (c.T)
@@ -684,7 +684,10 @@ int copy_k(Ctx &c, int32_t *k_out, uint32_t *tris_out)
 }
 
 // Autotuner: coordinate descent over the settings of the on-demand variant.
-// Every trial is a full run whose k is compared with the default run's.
+// Every trial is a full run whose k is compared with the default run's. The
+// settings are the list form's, so the trials run in it; sort_shift is tried in
+// the bit form where that is the form of the graph's runs and reads it. Where the
+// lists do not fit in memory, sort_shift alone is tried.
 int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_sec, double *default_sec)
 {
 	if (!c.dO)
@@ -696,9 +699,10 @@ int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_se
 	bool have_ref = false;
 	// one run under t, timed on the device (t_total); the first one sets the
 	// reference result
-	auto trial = [&](const nucleus34_tune &t, double &sec) -> int {
+	auto trial = [&](const nucleus34_tune &t, bool lists, double &sec) -> int {
 		c.tune_pinned = true;
 		c.tune_pin = t;
+		c.force_lists = lists;
 		nucleus34_result r{};
 		N34_TRY(run(c, NUCLEUS34_ONDEMAND, &r));
 		sec = r.t_total;
@@ -716,13 +720,34 @@ int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_se
 											  " changed the result");
 		return NUCLEUS34_OK;
 	};
+	// the default run's time, the better of two
+	auto time_default = [&](const nucleus34_tune &t, bool lists, double &sec) -> int {
+		double a = 0, b = 0;
+		N34_TRY(trial(t, lists, a));
+		N34_TRY(trial(t, lists, b));
+		sec = std::min(a, b);
+		return NUCLEUS34_OK;
+	};
 	auto body = [&]() -> int {
 		const nucleus34_tune def = tune_filled(nucleus34_tune{});
-		double s0 = 0, s1 = 0, s2 = 0;
-		N34_TRY(trial(def, s0)); // warm-up and reference
-		N34_TRY(trial(def, s1));
-		N34_TRY(trial(def, s2));
-		const double t_def = std::min(s1, s2);
+		double s0 = 0, t_rows = 0, t_def = 0;
+		N34_TRY(trial(def, false, s0)); // warm-up, reference and the form of the graph's runs
+		const bool rows = c.rows_run, rows_order = rows && c.T >= ORDER_MIN_TRIANGLES;
+		if (rows_order)
+			N34_TRY(time_default(def, false, t_rows));
+		bool lists = true;
+		const int rl = time_default(def, true, t_def);
+		if (rl == NUCLEUS34_E_OOM_BUDGET && rows)
+		{
+			clear_error();
+			lists = false;
+			if (rows_order)
+				t_def = t_rows;
+			else
+				N34_TRY(time_default(def, false, t_def));
+		}
+		else if (rl)
+			return rl;
 		nucleus34_tune best = def;
 		double t_best = t_def;
 		const uint32_t NEVER = NUCLEUS34_TUNE_NEVER;
@@ -741,6 +766,11 @@ int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_se
 								{&nucleus34_tune::sort_shift, &shifts},
 								{&nucleus34_tune::rounds_per_replay, &rounds}};
 		for (const Field &fd : fields)
+		{
+			const bool in_rows = rows_order && fd.f == &nucleus34_tune::sort_shift;
+			if (!in_rows && !lists)
+				continue;
+			double &t = in_rows ? t_rows : t_best;
 			for (uint32_t v : *fd.values)
 			{
 				if (best.*fd.f == v)
@@ -748,15 +778,18 @@ int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_se
 				nucleus34_tune cand = best;
 				cand.*fd.f = v;
 				double a = 0, b = 0;
-				N34_TRY(trial(cand, a));
-				if (a >= 0.99 * t_best)
+				N34_TRY(trial(cand, !in_rows, a));
+				if (a >= 0.99 * t)
 					continue;
-				N34_TRY(trial(cand, b)); // confirm: both runs 1% faster
-				if (b >= 0.99 * t_best)
+				N34_TRY(trial(cand, !in_rows, b)); // confirm: both runs 1% faster
+				if (b >= 0.99 * t)
 					continue;
 				best = cand;
-				t_best = 0.5 * (a + b);
+				t = 0.5 * (a + b);
 			}
+		}
+		if (!lists && rows_order)
+			t_best = t_rows;
 		if (best_out)
 			*best_out = best;
 		if (best_sec)
@@ -787,6 +820,7 @@ int autotune(Ctx &c, const char *path, nucleus34_tune *best_out, double *best_se
 	const int rc = body();
 	c.tune_pinned = pinned0;
 	c.tune_pin = pin0;
+	c.force_lists = false;
 	return rc;
 }
 

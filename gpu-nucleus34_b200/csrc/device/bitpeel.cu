@@ -561,7 +561,7 @@ bool bit_form_wanted(const Ctx &c, int variant)
 								   NUCLEUS34_OPT_NO_SMALL_ROUNDS | NUCLEUS34_OPT_FRONTIER_BY_C |
 								   NUCLEUS34_OPT_CHUNKED_DEBIT | NUCLEUS34_OPT_SCALAR_SCANS |
 								   NUCLEUS34_OPT_PIPELINED_DEBIT | NUCLEUS34_OPT_DEBIT_CURSOR;
-	return c.one_way && (variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM));
+	return c.one_way && !c.force_lists && (variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM));
 }
 
 // The rows are worth their words: every triangle's words are read in the support

@@ -89,6 +89,10 @@ struct PeelCtl
 	uint32_t error;      // nonzero: a device-side check failed (code)
 };
 
+// The bit-matrix and direct peels put frontiers in id order from this many
+// triangles on (see run_peel_loop).
+constexpr uint64_t ORDER_MIN_TRIANGLES = uint64_t(1) << 24;
+
 // Library context: one device, one stream, budgeted allocations.
 struct Ctx
 {
@@ -109,6 +113,8 @@ struct Ctx
 	uint32_t opt_flags = 0;
 	double peel_debit_sec = 0; // profiling only: debit kernels' device time
 	bool lean_run = false;     // this run uses the memory-lean layout
+	bool rows_run = false;     // this run uses the bit form
+	bool force_lists = false;  // runs use the list form (autotuner)
 	std::mutex mu;
 
 	// resident graph

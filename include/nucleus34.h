@@ -308,7 +308,12 @@ int nucleus34_ctx_last_tune(nucleus34_ctx ctx, nucleus34_tune *out);
 /* Autotuner for the uploaded graph: times its on-demand decomposition under
  * the defaults, then under candidate settings, one field at a time (each
  * field keeps the best value found before the next is tried; a candidate
- * must beat the best so far by 1% twice). Every run's k must equal the
+ * must beat the best so far by 1% twice). The settings are the list form's
+ * (see NUCLEUS34_OPT_PROFILE_PEEL), so the runs are of that form and the times
+ * are its times, also where the graph's own runs take the bit matrices;
+ * sort_shift, which these read from 2^24 triangles on, is then tried on them.
+ * Where the lists do not fit in memory the times are the bit form's and
+ * sort_shift alone is tried. Every run's k must equal the
  * default run's bit for bit (E_CUDA otherwise). The best settings go to
  * *best, their time and the default time (s, device-timed t_total) to
  * *best_sec and *default_sec, and, when path is non-NULL, into the table
