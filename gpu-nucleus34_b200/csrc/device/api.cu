@@ -293,12 +293,15 @@ int upload(Ctx &c, const nucleus34_csr *csr)
 // defaults. Called once T is known.
 void select_tune(Ctx &c, int variant)
 {
-	c.tune = tune_filled(nucleus34_tune{});
+	const nucleus34_tune defaults = tune_filled(nucleus34_tune{});
+	c.tune = defaults;
+	c.order_pinned = false;
 	if (variant != NUCLEUS34_ONDEMAND)
 		return;
 	if (c.tune_pinned)
 	{
 		c.tune = tune_filled(c.tune_pin);
+		c.order_pinned = c.tune.sort_shift != defaults.sort_shift;
 		return;
 	}
 	if (c.tune_rules.empty())

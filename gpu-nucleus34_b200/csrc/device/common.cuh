@@ -90,7 +90,7 @@ struct PeelCtl
 };
 
 // The bit-matrix and direct peels put frontiers in id order from this many
-// triangles on (see run_peel_loop).
+// triangles on, unless a pinned sort_shift asks for it (see run_peel_loop).
 constexpr uint64_t ORDER_MIN_TRIANGLES = uint64_t(1) << 24;
 
 // Library context: one device, one stream, budgeted allocations.
@@ -110,6 +110,7 @@ struct Ctx
 	bool tune_pinned = false;         // settings pinned by nucleus34_ctx_set_tune
 	nucleus34_tune tune_pin{};
 	nucleus34_tune tune = tune_filled(nucleus34_tune{}); // settings of the current / last run
+	bool order_pinned = false; // its sort_shift is pinned to another value than the default
 	uint32_t opt_flags = 0;
 	double peel_debit_sec = 0; // profiling only: debit kernels' device time
 	bool lean_run = false;     // this run uses the memory-lean layout

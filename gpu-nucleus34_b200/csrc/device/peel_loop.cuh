@@ -694,11 +694,11 @@ int run_peel_loop(Ctx &c, LoopBuffers &b, const Path &path, int32_t *S, int32_t 
 	// Frontiers are put in id order from T / 2^(sort_shift - 3) triangles on (an
 	// eighth of the list form's rule: the append buffers leave runs of
 	// neighbours), on graphs of 2^24 triangles and more, whose supports alone
-	// are as large as half of L2. Peel of R-MAT scale 18 (8.3e7 triangles) with
+	// are as large as half of L2, and wherever the caller pins a threshold. Peel of R-MAT scale 18 (8.3e7 triangles) with
 	// T/2^14, 2^12, 2^9, never: 176, 172, 170, 173 ms; geometric, 1.1e8: 53.4,
 	// 53.2, 52.9, 57.2; R-MAT scale 16 (1.6e7) 35.5, 35.5, 33.4, 32.0; geometric,
 	// 2e7: 9.8, 9.7, 9.6, 9.5.
-	if (tn.sort_shift != NUCLEUS34_TUNE_NEVER && c.T >= ORDER_MIN_TRIANGLES)
+	if (tn.sort_shift != NUCLEUS34_TUNE_NEVER && (c.T >= ORDER_MIN_TRIANGLES || c.order_pinned))
 		g.sort_min = uint32_t(std::max<uint64_t>(c.T >> (tn.sort_shift > 3 ? tn.sort_shift - 3 : 0), 4096));
 	// as many blocks as fit at once, fewer for small graphs, whose frontiers do
 	// not fill them (a quarter as many blocks: 19% slower on R-MAT scale 12; one

@@ -273,7 +273,8 @@ typedef struct
 	uint32_t sort_shift;        /* put a frontier of at least max(T >> sort_shift, 4096) triangles
 	                               in id order: 1..31 (default 12), or NUCLEUS34_TUNE_NEVER; the
 	                               bit-matrix and direct peels: 8T >> sort_shift, from 2^24
-	                               triangles on */
+	                               triangles on, below only if pinned to another
+	                               value than the default */
 	uint32_t rounds_per_replay; /* peel rounds per CUDA graph replay: 1..64 (default 16) */
 } nucleus34_tune;
 
