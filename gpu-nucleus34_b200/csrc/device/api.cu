@@ -6,6 +6,7 @@
 // their CSR upload (cuNucleus34.cu:290-293) is nucleus34_ctx_upload, their
 // phase timers (hrc::now() around synchronised phases) become CUDA events on
 // the library stream.
+#include "form.h"
 #include "pipeline.cuh"
 
 #include <algorithm>
@@ -350,7 +351,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	{
 		c.peel_debit_sec = 0;
 		N34_CUDA(cudaEventRecord(ev.e[0], c.stream));
-		if ((rc = list_triangles(c, rows ? &mats : nullptr, rows_least_triangles(c, variant))))
+		if ((rc = list_triangles(c, rows ? &mats : nullptr, rows_least_triangles(variant, c.m))))
 			break;
 		*lists = mats.cells != nullptr;
 		if (mats.cells)

@@ -39,6 +39,7 @@
 
 #include <algorithm>
 
+#include "form.h"
 #include "peel_loop.cuh"
 
 namespace n34 {
@@ -564,37 +565,6 @@ bool bit_form_wanted(const Ctx &c, int variant)
 	return c.one_way && !c.force_lists && (variant == NUCLEUS34_DIRECT || !(c.opt_flags & LIST_FORM));
 }
 
-// The rows are worth their words: every triangle's words are read in the support
-// count and once more when it dies, however few bits they hold, where the lists
-// cost by what they hold. `lists` is the lesser of the entries on the triangles'
-// head and tail edges (those with the edge as head or tail: the others are not
-// counted before the in-rows are built). Words and entries of R-MAT and geometric
-// graphs are 0.1 to 1.1 to one. Hubs that are joined to each other and to many
-// vertices of degree 1 to 3 (in-rows long and nearly empty) cross over between
-// 2.9 and 4.7 on demand, where the lists' rounds take longer (incidence, support
-// and peel, rows against lists, ms: 8.1 and 14.1 at 1.1, 14.7 and 15.6 at 2.9,
-// 20.5 and 15.6 at 4.7, 94 and 33 at 26), and between 1.5 and 2 in the direct
-// variant, which peels over the clique list in either form (19.7 and 25 at 1.5,
-// 19.0 and 15.5 at 2.0, 237 and 32 at 26). On demand the lists also take 1 to 2
-// ms for the launches of their rounds: the time of 1e8 words.
-static bool rows_pay(int variant, uint64_t words, uint64_t lists)
-{
-	return variant == NUCLEUS34_DIRECT ? words <= lists + lists / 2 : words <= 3 * lists + lists / 2 + 100000000;
-}
-
-// From this many triangles on the listing keeps its matrices: building in-rows is
-// several passes over the edges, whatever the triangles. On demand that is 0.03
-// ns an edge against 1 ms for the launches of the lists' rounds (if any: road-like
-// grids have no cliques); the direct variant also sorts the in-edges, 0.2 ns an
-// edge, and has no such launches. Incidence, support, cliques and peel, rows against
-// lists, ms: on demand, 2e6 edges and 2e5 triangles 0.25 and 0.26, 3.2e7 and 6e5
-// 1.86 and 0.98, 1.2e7 and 4e4 (with rounds) 1.2 and 1.5; direct, 8e6 and 1.5e6
-// 2.0 and 1.3, 6e6 and 3.5e6 2.76 and 2.81, 1e7 and 1e7 5.7 and 7.4.
-uint64_t rows_least_triangles(const Ctx &c, int variant)
-{
-	return variant == NUCLEUS34_DIRECT ? c.m / 2 : c.m > (uint64_t(1) << 23) ? c.m / 16 : 0;
-}
-
 int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fits)
 {
 	const uint64_t T = c.T, m = c.m;
@@ -644,11 +614,8 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fi
 		}
 		c.release(indeg);
 		indeg = nullptr;
-		// the in-rows and their triangles, the counts; then support, k, two
-		// frontiers, the ordering bitmap and, if kept, the death rounds
 		const uint64_t room = c.budget > c.in_use ? c.budget - c.in_use : 0;
-		const uint64_t per_tri = c.opt_flags & NUCLEUS34_OPT_VERIFIABLE ? 24 : 20;
-		if (in.nwords > 0xffffffffull || 16 * in.nwords + per_tri * T + T / 8 + 16 * m + (uint64_t(1) << 20) > room)
+		if (!rows_fit(in.nwords, T, m, c.opt_flags & NUCLEUS34_OPT_VERIFIABLE, room))
 			break;
 		if ((rc = dalloc(c, &in.cells, in.nwords, "in-rows")) || (rc = dalloc(c, &in.live, m, "in-row counts")))
 			break;

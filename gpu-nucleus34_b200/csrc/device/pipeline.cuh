@@ -104,8 +104,6 @@ bool bit_form_wanted(const Ctx &c, int variant);
 // the form needs beside them exceed the room left, or when the lists are the less
 // work. In the direct variant columns ascend with the in-edge's source (by_source).
 int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fits);
-// Fewest triangles from which on the form may pay.
-uint64_t rows_least_triangles(const Ctx &c, int variant);
 void free_in_rows(Ctx &c, InMats &in);
 // own (optional, needs by_source): cliques whose lowest triangle is t. *acyclic:
 // no three vertices above one source form a directed cycle (the rows would take
