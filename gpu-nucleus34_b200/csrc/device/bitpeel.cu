@@ -83,27 +83,31 @@ __global__ void k_in_sorted_columns(const uint32_t *__restrict__ E, const unsign
 struct EdgeSums
 {
 	unsigned long long sum_sq;  // of the triangles on an edge (k_in_counts)
-	unsigned long long words;   // row and in-row words of all triangles
-	unsigned long long heads;   // sum over triangles of the triangles whose head or tail edge is
-	unsigned long long tails;   // theirs: of their head edge, of their tail edge
+	// row and in-row words of all triangles; the triangles that have a triangle's
+	// head edge as head or tail, over all triangles; those that have its tail edge
+	unsigned long long words, heads, tails;
 };
 
-// v of all threads of the block to *sum (all threads call)
-__device__ __forceinline__ void block_sum(unsigned long long v, unsigned long long *sum)
+// v[i] of all threads of the block to sum[i] (all threads call)
+template <int N>
+__device__ __forceinline__ void block_sums(unsigned long long (&v)[N], unsigned long long *sum)
 {
-	__shared__ unsigned long long s_sum;
-	if (threadIdx.x == 0)
-		s_sum = 0;
+	__shared__ unsigned long long s_sum[N];
+	if (threadIdx.x < N)
+		s_sum[threadIdx.x] = 0;
 	__syncthreads();
 #pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		v += __shfl_xor_sync(FULL, v, o);
-	if (lane_id() == 0 && v)
-		atomicAdd(&s_sum, v);
+	for (int i = 0; i < N; ++i)
+	{
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1)
+			v[i] += __shfl_xor_sync(FULL, v[i], o);
+		if (lane_id() == 0 && v[i])
+			atomicAdd(s_sum + i, v[i]);
+	}
 	__syncthreads();
-	if (threadIdx.x == 0 && s_sum)
-		atomicAdd(sum, s_sum);
-	__syncthreads();
+	if (threadIdx.x < N && s_sum[threadIdx.x])
+		atomicAdd(sum + threadIdx.x, s_sum[threadIdx.x]);
 }
 
 // cells of every edge's in-row; cnt: triangles whose head or tail edge it is
@@ -111,7 +115,7 @@ __global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const 
 							const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
 							uint32_t *__restrict__ width, uint32_t *__restrict__ cnt, EdgeSums *__restrict__ sums)
 {
-	unsigned long long words = 0, heads = 0, tails = 0;
+	unsigned long long acc[3] = {0, 0, 0}; // words, heads, tails
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
 	{
@@ -126,13 +130,11 @@ __global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const 
 		}
 		width[e] = in;
 		cnt[e] = sym;
-		words += uint64_t(head) * (W + in);
-		heads += uint64_t(head) * sym;
-		tails += uint64_t(sym - head) * sym;
+		acc[0] += uint64_t(head) * (W + in);
+		acc[1] += uint64_t(head) * sym;
+		acc[2] += uint64_t(sym - head) * sym;
 	}
-	block_sum(words, &sums->words);
-	block_sum(heads, &sums->heads);
-	block_sum(tails, &sums->tails);
+	block_sums(acc, &sums->words);
 }
 
 __global__ void k_in_starts(const uint64_t *__restrict__ off, uint64_t m, uint4 *__restrict__ erec)
@@ -160,7 +162,7 @@ __global__ void k_in_counts(const uint4 *__restrict__ erec, uint64_t m, const ui
 							const uint32_t *__restrict__ width, uint32_t *__restrict__ cnt,
 							uint2 *__restrict__ live, unsigned long long *__restrict__ sum_sq)
 {
-	unsigned long long acc = 0;
+	unsigned long long acc[1] = {0};
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
 	{
@@ -171,9 +173,9 @@ __global__ void k_in_counts(const uint4 *__restrict__ erec, uint64_t m, const ui
 		const unsigned long long d = uint64_t(n) + rest;
 		cnt[e] = n;
 		live[e] = make_uint2(n, W);
-		acc += d * d;
+		acc[0] += d * d;
 	}
-	block_sum(acc, sum_sq);
+	block_sums(acc, sum_sq);
 }
 
 // first positions of the cells' triangles in tri; all not dead, none dying. A
