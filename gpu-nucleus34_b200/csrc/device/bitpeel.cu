@@ -470,7 +470,7 @@ struct BitPath
 		Settler found(*this, m, g, Fn, slot, level);
 		const uint32_t lane = lane_id();
 		const Units u = debit_units(nF, loop_warps());
-		claim_units(u.total, &slot->work, [&](uint32_t unit) {
+		claim_units(u.total, &slot->work, &g.ctl->c.error, [&](uint32_t unit) {
 			// of the warps that share a triangle, half take its rows and half its
 			// in-rows (R-MAT scale 12: 3% less than one after the other)
 			const uint32_t shift = u.shift ? u.shift - 1 : 0u;

@@ -51,7 +51,7 @@ struct DirectPath
 		Appender next{m.next, Fn, &slot->n, &g.ctl->c.error, g.T, 0u};
 		const uint32_t lane = lane_id();
 		const Units u = debit_units(nF, loop_warps());
-		claim_units(u.total, &slot->work, [&](uint32_t unit) {
+		claim_units(u.total, &slot->work, &g.ctl->c.error, [&](uint32_t unit) {
 			const uint32_t stripe = unit & ((1u << u.shift) - 1u);
 			const uint32_t base = (unit >> u.shift) * u.ch;
 			uint32_t t = 0, len = 0;

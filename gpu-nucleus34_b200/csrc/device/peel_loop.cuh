@@ -43,6 +43,8 @@ constexpr uint32_t NO_SUPPORT = 0xffffffffu;
 constexpr unsigned long long LOOP_WAIT_LIMIT_NS = 60ull * 1000000000ull;
 constexpr unsigned long long LOOP_TIME_LIMIT_NS = 600ull * 1000000000ull;
 
+constexpr uint32_t CLAIM_TRIES = 1u << 24; // of 32 ns or more
+
 struct alignas(16) PhaseSlot
 {
 	uint32_t arrived; // blocks at the phase's barrier
@@ -273,7 +275,7 @@ __device__ __forceinline__ Units debit_units(uint32_t nF, uint32_t nwarps)
 // direct, 8.84 -> 8.59 ms, scale 12 3.89 -> 3.79 and 10, direct, 1.63 -> 1.56,
 // scale 16 31.4 -> 31.2.
 template <class Fn>
-__device__ __forceinline__ void claim_units(uint32_t total, uint32_t *work, Fn &&f)
+__device__ __forceinline__ void claim_units(uint32_t total, uint32_t *work, uint32_t *err, Fn &&f)
 {
 	const uint32_t nwarps = loop_warps();
 	if (total <= nwarps)
@@ -322,9 +324,16 @@ __device__ __forceinline__ void claim_units(uint32_t total, uint32_t *work, Fn &
 					unit = b;
 					break;
 				}
-				// another warp is fetching it
-				while ((uint32_t)(*(volatile unsigned long long *)&s_range >> 32) == end)
+				// another warp is fetching it: one atomic's round trip. After a second
+				// or so the call ends with an error instead.
+				uint32_t tries = 0;
+				while ((uint32_t)(*(volatile unsigned long long *)&s_range >> 32) == end && ++tries < CLAIM_TRIES)
 					__nanosleep(32);
+				if (tries >= CLAIM_TRIES)
+				{
+					atomicOr(err, 1u);
+					break;
+				}
 			}
 		}
 		unit = __shfl_sync(FULL, unit, 0);
