@@ -798,34 +798,37 @@ def main():
     return 0
 
 
-def roofline(r, prof, peaks, kind):
-    """HBM roofline of the two intersection phases.
+# Atomics with a result on 32 MB that stay in L2, one B200 (a separate measurement;
+# on 320 MB 2.8e10): the rate that bounds the debit's support updates.
+L2_ATOMICS_PER_S = 1.25e11
 
-    Algorithmic bytes of one full enumeration (every triangle's lists
-    intersected once) use the zipper bound 4*sum_e T(e)^2 + 36*T + 48*Q: each
-    triangle reads its three edges' incidence lists (4 B per entry), its own
-    record and list bounds (36 B), and each of the 4Q clique occurrences reads
-    3 partner ids (48 B per clique). The support count performs one
-    enumeration in one launch (k_support_bits); the peel performs it once more,
-    spread over the debit phases of its one launch (k_peel_loop), which the
-    kernel times itself in a separate run of the same workload. Both read bit
-    rows in place of lists (32 candidates per 16 bytes), so they move far fewer
-    bytes than this bound and a fraction above 1 is possible. traffic is null:
-    no capture of these kernels at this size was taken."""
-    T, Q, S2 = r["triangle_count"], r["four_clique_count"], r["sum_te_sq"]
-    alg = 4 * S2 + 36 * T + 48 * Q
-    peak = peaks.get("hbm_gbs")
+
+def roofline(r, prof, peaks, kind):
+    """Bounds of the two kernels that carry the time.
+
+    The debit phases of the peel's one launch (k_peel_loop; their time comes from
+    the kernel itself, in a separate run of the same workload) must update the
+    supports of the partners of every clique that dies, at most 3Q atomics: the
+    bound is the rate of L2 atomics. The rows they read stay in L2 for the most
+    part, so HBM bytes bound nothing. The support count (k_support_bits, one
+    launch) must read every triangle's record and write its support, 16T bytes;
+    its rows are read again and again from L1 and L2, and are not counted. traffic
+    is null: no capture of these kernels at this size was taken."""
+    T, Q = r["triangle_count"], r["four_clique_count"]
+    hbm = peaks.get("hbm_gbs")
     pk = f"{kind} ({'hbm_gbs' if kind == 'measured' else 'fallback 6.65 TB/s'})"
-    out = []
-    for name, t, launches, what in (
-            ("k_peel_loop", prof.get("t_peel_debit", 0.0), 1, "debit phases of the peel, all rounds (profiling run)"),
-            ("k_support_bits", r["t_support"], 1, "support count (one launch, timed run)")):
-        ach = alg / t / 1e9 if t > 0 else None
-        out.append({"kernel": name, "what": what, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
-                    "frac": (ach / peak) if (ach and peak) else None,
-                    "traffic": None, "algorithmic_bytes": alg,
-                    "device_seconds": t, "launches": launches, "peak_kind": pk,
-                    "definition": "4*sum_e T(e)^2 + 36T + 48Q bytes per full enumeration (zipper bound)"})
+
+    def entry(kernel, what, bound, work, t, peak, unit, peak_kind, definition):
+        ach = work / t / 1e9 if t > 0 else None
+        return {"kernel": kernel, "what": what, "bound": bound, "achieved": ach, "peak": peak, "unit": unit,
+                "frac": (ach / peak) if (ach and peak) else None, "traffic": None, "algorithmic_work": work,
+                "device_seconds": t, "launches": 1, "peak_kind": peak_kind, "definition": definition}
+
+    out = [entry("k_peel_loop", "debit phases of the peel, all rounds (profiling run)", "l2 atomics", 3 * Q,
+                 prof.get("t_peel_debit", 0.0), L2_ATOMICS_PER_S / 1e9, "G atomics/s",
+                 "measured (atomics with a result on 32 MB)", "3Q support updates"),
+           entry("k_support_bits", "support count (one launch, timed run)", "hbm", 16 * T, r["t_support"], hbm, "GB/s",
+                 pk, "16T bytes: triangle records read, supports written")]
     # the dominant kernel is the one with the larger device time
     if out[1]["device_seconds"] > out[0]["device_seconds"]:
         out.reverse()

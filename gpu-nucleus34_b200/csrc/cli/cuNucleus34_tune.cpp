@@ -2,8 +2,9 @@
 // the dataset's graph class (nucleus34_ctx_autotune) and writes the fastest
 // settings into the table, which cuNucleus34_ondemand then reads from
 // NUCLEUS34_TUNE_TABLE. Prints one JSON line: the class, the settings and the
-// device times of the default and the tuned decomposition, and of a last
-// unpinned run that takes its settings from the table. Exit code 1 on any
+// device times of the default and the tuned decomposition in the list form,
+// whose settings they are (nucleus34_ctx_autotune), and of a last unpinned run in
+// the form that the graph takes, with its settings from the table. Exit code 1 on any
 // error (the JSON then holds "error").
 #include <cstdint>
 #include <cstdio>

@@ -30,7 +30,7 @@
 // the others. On one B200 atomics with a result run at 1.25e11 per second on
 // 32 MB, 2.8e10 on 320 MB (loads of 4 bytes: 2.7e11, 5.8e10; of 16 bytes:
 // 1.4e11, 3.8e10), so R-MAT scale 18's 2.3e9 cliques take 129 ms of its peel's
-// 167. Hence: state bits beside the ids in the cell (one gather tells both; a
+// 164. Hence: state bits beside the ids in the cell (one gather tells both; a
 // separate word cost 330 ms), no loads of supports that other warps debit, and
 // row words that leave out what a dying partner of lower id owns (2.3e9
 // cliques settled instead of 3.8e9). A pipeline of asynchronous copies that kept

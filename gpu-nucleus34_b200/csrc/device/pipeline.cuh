@@ -25,11 +25,12 @@ struct Incidence
 constexpr uint32_t INC_DEAD = 0x80000000u;
 // Most triangles the on-demand peel keeps its death flags in the incidence
 // for (ids leave the top two bits of a tri word free); above it the slower
-// round-stamp peel runs. Union passes (batched form, serving) are cut below it.
+// round-stamp peel runs. Union passes (batched form, serving) are cut below it,
+// as a pass may have to run on the lists; the bit form itself has no such limit.
 constexpr uint64_t FLAG_PEEL_MAX_TRIANGLES = 0x3fffffffull;
 
-// The triangle listing's bit matrices, kept for the on-demand variant. Source
-// u of out-degree d has a d x d matrix of W = ceil(d / 32) cells per row. Row
+// The triangle listing's bit matrices, kept for the bit form of both variants.
+// Source u of out-degree d has a d x d matrix of W = ceil(d / 32) cells per row. Row
 // ia belongs to edge O[u] + ia, so an edge stands for its row.
 struct BitMats
 {

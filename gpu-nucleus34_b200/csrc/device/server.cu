@@ -225,7 +225,8 @@ void worker_loop(nucleus34_server_s *s, size_t wi)
 	Slot &slot = s->slots[s->worker_slot[wi]];
 	cudaSetDevice(c.device);
 	const uint64_t range_limit = 0xffffffffull / 3; // 3T incidence entries in 32-bit positions
-	// on-demand unions stay within the death-flag peel's triangle range
+	// on-demand unions stay within the triangle range of the death flags, which
+	// the list form keeps
 	const uint64_t ondemand_limit = std::min(range_limit, FLAG_PEEL_MAX_TRIANGLES);
 	const uint64_t clique_limit = 0xffffffffull;     // direct: clique ids in 32 bits
 	for (;;)

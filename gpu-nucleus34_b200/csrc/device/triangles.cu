@@ -25,8 +25,8 @@
 //               and B position pb is triangle (O[u]+ia, b, O[v]+pb), and its
 //               canonical position is the row word's first id + the set bits
 //               of the word below ib. No search is needed for c.
-// The matrices can be kept (BitMats) for the on-demand variant's support count
-// and peel (bitpeel.cu).
+// The matrices can be kept (BitMats) for the support count, the clique list and
+// the peel on them (bitpeel.cu, bitcliques.cu).
 // Steps 1-2 hold 12 bytes per (column, row tile) of each source; when
 // those do not fit the budget the sources are taken in chunks, counting all
 // of them first and repeating steps 1-2 before each chunk's writes. The kept

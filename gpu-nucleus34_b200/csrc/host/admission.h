@@ -23,11 +23,13 @@ constexpr uint64_t PASS_BYTES_PER_TRIANGLE = 80;
 constexpr uint64_t PASS_BYTES_PER_EDGE = 40;
 constexpr uint64_t DIRECT_BYTES_PER_CLIQUE = 33;
 
-// Direct share of a slot's budget (1/64). Alone, a graph is decomposed
-// faster by the direct variant up to about 1e8 four-cliques, but a direct
-// union of many such graphs streams its clique list from DRAM where the
-// graph alone kept it in L2: on the full serving mix (edges up to 1e7) a
-// share of 1/8 served 13.3-13.7 graphs/s, 1/64 14.2 and on-demand only 14.3.
+// Direct share of a slot's budget (1/64). The two variants differ little up to
+// about 1e7 four-cliques (alone, direct 0.85 to 1.14 times as fast); beyond, a
+// direct pass does the same work on the same rows and writes its clique list
+// besides (0.67 to 0.86 times as fast). On the full serving mix (2000 requests,
+// edges up to 1e7, four times the serial rate) a share of 1/8 (1634 requests
+// direct) served 27.9 graphs/s, 1/64 (1285) 30.9 and 31.3, on-demand only 29.9 and
+// 31.2.
 constexpr uint32_t DEFAULT_DIRECT_DIV = 64;
 
 // Out-wedges sum_u C(d, 2) (bound on the triangles) and out-triples

@@ -75,8 +75,9 @@ typedef struct
 	uint32_t flags;            /* NUCLEUS34_OPT_* bits, 0 = defaults */
 } nucleus34_opts;
 
-/* opts.flags: force the round-stamp ownership test in the on-demand peel
- * (the default keeps death flags inside the incidence entries when T < 2^30). */
+/* opts.flags: the list form of the on-demand peel with the round-stamp
+ * ownership test (its default keeps death flags inside the incidence entries
+ * when T < 2^30). */
 #define NUCLEUS34_OPT_STAMP_PEEL 0x1u
 /* opts.flags: print the peel's device time per step (mark, debit, level scan,
  * frontier order) to stderr and return the debit's in t_peel_debit. With a
@@ -85,11 +86,15 @@ typedef struct
 #define NUCLEUS34_OPT_PROFILE_PEEL 0x2u
 /* The on-demand variant peels on the triangle listing's bit matrices, all
  * rounds in one cooperative launch; so does the direct variant, on its clique
- * list up to 2^24 cliques. The list form, on the incidence lists, serves graphs whose matrices do
- * not fit in the memory budget, and the flags below that select a layout or a
- * schedule of it (STAMP_PEEL, LEAN_MEMORY, HOST_LOOP, NO_SMALL_ROUNDS,
- * FRONTIER_BY_C, CHUNKED_DEBIT, SCALAR_SCANS, PIPELINED_DEBIT, DEBIT_CURSOR;
- * they do not concern the direct variant). Results are identical. */
+ * list up to 2^24 cliques. The list form, on the incidence lists, serves graphs
+ * whose matrices do not fit in the memory budget (or, in a serving pass, in what
+ * the pass was admitted with) or exceed their 16- and 32-bit positions, graphs on
+ * which it is the less work (long, nearly empty rows; few triangles among many
+ * edges), CSRs with directed cycles or edges in both directions, and the flags
+ * below that select a layout or a schedule of it (STAMP_PEEL, LEAN_MEMORY,
+ * HOST_LOOP, NO_SMALL_ROUNDS, FRONTIER_BY_C, CHUNKED_DEBIT, SCALAR_SCANS,
+ * PIPELINED_DEBIT, DEBIT_CURSOR; they do not concern the direct variant).
+ * Results are identical. */
 /* opts.flags: the memory-lean layout of the list form (T < 2^30):
  * incidence entries sorted in place (no 64-bit sort keys beside them), no
  * per-triangle entry positions (the peel searches for a triangle's entries),
