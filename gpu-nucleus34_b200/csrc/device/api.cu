@@ -346,14 +346,15 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	uint32_t *own = nullptr;
 	int rc = NUCLEUS34_OK;
 	PeelCtl pc{};
-	bool peeled = false, acyclic = true;
+	bool peeled = false, acyclic = true, rows_used = false;
+	*lists = false;
 	do
 	{
 		c.peel_debit_sec = 0;
 		N34_CUDA(cudaEventRecord(ev.e[0], c.stream));
 		if ((rc = list_triangles(c, rows ? &mats : nullptr, rows_least_triangles(variant, c.m))))
 			break;
-		*lists = mats.cells != nullptr;
+		rows_used = mats.cells != nullptr;
 		if (mats.cells)
 			budget.limit();
 		if ((rc = segments_after_listing(c)))
@@ -382,7 +383,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 			free_mats(c, mats);
 			budget.lift();
 		}
-		*lists = c.rows_run = bits;
+		rows_used = c.rows_run = bits;
 		if (bits)
 			r.sum_te_sq = in.sum_te_sq;
 		else if (c.T)
@@ -492,7 +493,7 @@ static int run_phases(Ctx &c, int variant, bool rows, bool *lists, nucleus34_res
 	free_in_rows(c, in);
 	c.release(S);
 	c.release(own);
-	*lists = *lists && (rc == NUCLEUS34_E_OOM_BUDGET || !acyclic);
+	*lists = rows_used && (rc == NUCLEUS34_E_OOM_BUDGET || !acyclic);
 	if (rc)
 	{
 		c.release_results();
