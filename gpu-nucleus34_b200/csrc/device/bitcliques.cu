@@ -142,19 +142,8 @@ __global__ void __launch_bounds__(CL_THREADS) k_support_bits(
 			own[t] = mine;
 		acc += cnt;
 	}
-	unsigned long long row_acc = rowcnt;
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-	{
-		acc += __shfl_xor_sync(FULL, acc, o);
-		row_acc += __shfl_xor_sync(FULL, row_acc, o);
-	}
-	if (lane_id() == 0 && acc)
-	{
-		atomicAdd(total, acc);
-		if (row_acc)
-			atomicAdd(total + 1, row_acc);
-	}
+	unsigned long long sums[2] = {acc, rowcnt};
+	block_sums(sums, total);
 }
 
 __device__ __forceinline__ void sort2(uint32_t &a, uint32_t &b)

@@ -86,36 +86,15 @@ struct EdgeSums
 	// row and in-row words of all triangles; the triangles that have a triangle's
 	// head edge as head or tail, over all triangles; those that have its tail edge
 	unsigned long long words, heads, tails;
+	unsigned long long cells; // of the in-rows
 };
-
-// v[i] of all threads of the block to sum[i] (all threads call)
-template <int N>
-__device__ __forceinline__ void block_sums(unsigned long long (&v)[N], unsigned long long *sum)
-{
-	__shared__ unsigned long long s_sum[N];
-	if (threadIdx.x < N)
-		s_sum[threadIdx.x] = 0;
-	__syncthreads();
-#pragma unroll
-	for (int i = 0; i < N; ++i)
-	{
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1)
-			v[i] += __shfl_xor_sync(FULL, v[i], o);
-		if (lane_id() == 0 && v[i])
-			atomicAdd(s_sum + i, v[i]);
-	}
-	__syncthreads();
-	if (threadIdx.x < N && s_sum[threadIdx.x])
-		atomicAdd(sum + threadIdx.x, s_sum[threadIdx.x]);
-}
 
 // cells of every edge's in-row; cnt: triangles whose head or tail edge it is
 __global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const uint32_t *__restrict__ indeg,
 							const uint4 *__restrict__ erec, const uint4 *__restrict__ rows,
 							uint32_t *__restrict__ width, uint32_t *__restrict__ cnt, EdgeSums *__restrict__ sums)
 {
-	unsigned long long acc[3] = {0, 0, 0}; // words, heads, tails
+	unsigned long long acc[4] = {0, 0, 0, 0}; // words, heads, tails, cells
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
 	{
@@ -133,6 +112,7 @@ __global__ void k_in_widths(const uint32_t *__restrict__ src, uint64_t m, const 
 		acc[0] += uint64_t(head) * (W + in);
 		acc[1] += uint64_t(head) * sym;
 		acc[2] += uint64_t(sym - head) * sym;
+		acc[3] += in;
 	}
 	block_sums(acc, &sums->words);
 }
@@ -594,13 +574,13 @@ int build_in_rows(Ctx &c, const BitMats &mats, InMats &in, int variant, bool *fi
 		c.launches += 2;
 		if ((rc = scan_u32(c, width, off, m)))
 			break;
-		if (cudaMemcpyAsync(&in.nwords, off + m, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-			cudaMemcpyAsync(&hsums, sums, sizeof(EdgeSums), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+		if (cudaMemcpyAsync(&hsums, sums, sizeof(EdgeSums), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
 			cudaStreamSynchronize(c.stream) != cudaSuccess)
 		{
 			rc = fail(NUCLEUS34_E_CUDA, "in-row widths");
 			break;
 		}
+		in.nwords = hsums.cells;
 		if (!rows_pay(variant, hsums.words, std::min(hsums.heads, hsums.tails)))
 			break;
 		if (by_source)

@@ -70,6 +70,29 @@ __device__ __forceinline__ uint32_t warp_append(bool pred, uint32_t *counter)
 	return base + __popc(mask & lanemask_lt());
 }
 
+// v[i] of all threads of the block to sum[i], one atomic each per block (all threads
+// call; atomics of all warps on one address take about 1 ns each, whole GPU)
+template <int N>
+__device__ __forceinline__ void block_sums(unsigned long long (&v)[N], unsigned long long *sum)
+{
+	__shared__ unsigned long long s_sum[N];
+	if (threadIdx.x < N)
+		s_sum[threadIdx.x] = 0;
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < N; ++i)
+	{
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1)
+			v[i] += __shfl_xor_sync(FULL, v[i], o);
+		if (lane_id() == 0 && v[i])
+			atomicAdd(s_sum + i, v[i]);
+	}
+	__syncthreads();
+	if (threadIdx.x < N && s_sum[threadIdx.x])
+		atomicAdd(sum + threadIdx.x, s_sum[threadIdx.x]);
+}
+
 // Peel control block (device resident; one per run).
 struct PeelCtl
 {

@@ -41,7 +41,7 @@ struct BitMats
 	// w: symmetric, zero at first; the peel sets both when it begins to die.
 	// One 16-byte load tells a triangle's id and state.
 	uint4 *cells = nullptr;
-	// per oriented edge: {first cell of its row, W << 16 | its position in
+	// per oriented edge, in the same allocation: {first cell of its row, W << 16 | its position in
 	// N+(u), first cell of its in-row, its column among its head's in-edges}
 	uint4 *erec = nullptr;
 	uint64_t nwords = 0;

@@ -425,8 +425,7 @@ cudaError_t launch_tri_write(const uint32_t *O, const uint32_t *E, uint64_t n, c
 
 void free_mats(Ctx &c, BitMats &mats)
 {
-	c.release(mats.cells);
-	c.release(mats.erec);
+	c.release(mats.cells); // and the edge records behind them
 	mats = BitMats{};
 }
 
@@ -454,7 +453,6 @@ int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min)
 		c.release(cols);
 		c.release(rows);
 		c.release(cells);
-		c.release(erec);
 		c.release(err);
 	};
 	do
@@ -583,15 +581,16 @@ int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min)
 		if ((rc = dalloc(c, &c.dtris, 3 * T, "triangles")))
 			break;
 		bool kept = keep && T >= keep_min && nchunks == 1 && nwords <= 0xffffffffull && c.max_out <= 0xffffu &&
-					c.in_use + 16 * (m + alloc_w) + 512 <= c.rows_budget;
-		if (kept && (dalloc(c, &erec, m, "edge records") || dalloc(c, &cells, alloc_w, "listing cells")))
+					c.in_use + 16 * (m + alloc_w) + 256 <= c.rows_budget;
+		// one block: an allocation costs a small graph's call 4 us
+		if (kept && dalloc(c, &cells, alloc_w + m, "listing cells, edge records"))
 		{
-			c.release(erec);
-			erec = nullptr;
 			cells = nullptr;
 			kept = false;
 			clear_error();
 		}
+		if (kept)
+			erec = cells + alloc_w;
 		for (size_t i = 0; i < nchunks && !rc; ++i)
 		{
 			// a single chunk still holds its bits from the count
@@ -628,7 +627,6 @@ int list_triangles(Ctx &c, BitMats *keep, uint64_t keep_min)
 		{
 			*keep = BitMats{cells, erec, nwords};
 			cells = nullptr;
-			erec = nullptr;
 		}
 	} while (false);
 	cleanup();
